@@ -62,12 +62,14 @@ __global__ void __launch_bounds__(kBatchZT, 3) batch_pass_a(BatchDev b) {
                 const RectZoneIn in(b.a, cur, z, tile.nzx, z - tile.zo, tile.po);
                 pass_a_zone_thread<4>(b.a, c, in, dt, z, 4 * z, v, nbad);
             } else if (kAllQuads || tile.quads) {
-                pass_a_zone_thread<4>(b.a, c, cur, dt, z, 4 * z, v, nbad);
+                const GlobalZoneIn in{b.a, cur, z, 4 * z};
+                pass_a_zone_thread<4>(b.a, c, in, dt, z, 4 * z, v, nbad);
             } else {
                 const int n = b.a.znump[z];
                 const int64_t s0 = b.a.zfirst[z];
-                if (n == 4) pass_a_zone_thread<4>(b.a, c, cur, dt, z, s0, v, nbad);
-                else pass_a_zone_thread<3>(b.a, c, cur, dt, z, s0, v, nbad);
+                const GlobalZoneIn in{b.a, cur, z, s0};
+                if (n == 4) pass_a_zone_thread<4>(b.a, c, in, dt, z, s0, v, nbad);
+                else pass_a_zone_thread<3>(b.a, c, in, dt, z, s0, v, nbad);
             }
             fold = dmin(fold, v);
         }

@@ -304,7 +304,12 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
         cudaError_t e = prepare_pass_c(p.precision != PNT_PREC_FP64, a.quads != 0, a.rect_nzx, a.numz, nsm, &a.gridC);
         if (e != cudaSuccess) return fail(PNT_ERR_CUDA, "pass C setup: %s", cudaGetErrorString(e));
-        if (a.rect_nzx > 0 && p.precision != PNT_PREC_FP64) {
+        if (p.precision == PNT_PREC_FP64) {
+            int32_t ntiles = 0;
+            e = prepare_pass_a_fp64(a.rect_nzx, a.quads != 0, a.numz, nsm, &a.gridA, &ntiles);
+            if (e != cudaSuccess) return fail(PNT_ERR_CUDA, "pass A setup: %s", cudaGetErrorString(e));
+            if (pnt_status st = h->alloc(&a.redo, (size_t)ntiles)) return st;
+        } else if (a.rect_nzx > 0) {
             e = prepare_pass_a_rows_mixed(p.precision == PNT_PREC_LEARNED, a.rect_nzx, a.numz, nsm, &a.gridA);
             if (e != cudaSuccess) return fail(PNT_ERR_CUDA, "pass A setup: %s", cudaGetErrorString(e));
         }

@@ -17,15 +17,9 @@
 // Passes A and C add their blocks' dt minimum, dV/V maximum and inverted
 // sides to the cycle's reductions with atomics (exact in any order).
 //
-// Pass A runs one thread per zone (pass_a_zone_thread): the zone's sides
-// in the reference's side order, each zone-level quantity (centre, sums,
-// EOS) formed once, no shuffles, scheduled so the side arrays die early;
-// 128 registers, 4 blocks of 128 per SM.  It is bound by its ~2400
-// instructions per zone, a third of them the correctly rounded FP64
-// divisions and square roots; quotients whose IEEE result is fixed without
-// the division (zero over a finite non-zero divisor, division by one, the
-// zkur square root of a corner without compression) skip it, which a
-// quiescent region (zero velocities and pressure) hits on most corners.
+// Pass A runs one thread per zone: the zone's sides in the reference's side
+// order, each zone-level quantity (centre, sums, EOS) formed once, no
+// shuffles, its quotients and roots in straight-line code (ieee_div.cuh).
 // Pass C is the persistent staged kernel of pass_c.cu (one
 // thread per zone, inputs gathered into shared memory by asynchronous
 // copies); the batched kernels run the same two bodies.  1/elen is formed
@@ -38,44 +32,118 @@
 #include "hydro_fp64_body.cuh"
 
 #include <algorithm>
-#include "zone_tiles.cuh"
+#include "zone_stage.cuh"
 
 namespace pnt {
 namespace {
 
 using namespace fp64;
 
-#ifndef PNT_PASS_A_ZT_MIN_BLOCKS
-#define PNT_PASS_A_ZT_MIN_BLOCKS 4
-#endif
-constexpr int kZoneThreadsZT = 128;   // one zone per thread
+// Pass A: one warp a CTA, 8 an SM, each walking tiles of 32 zones (tiles
+// blockIdx.x, blockIdx.x + gridDim.x, ...) through its two stages
+// (zone_stage.cuh).  Zones that the straight-line body refuses are noted in
+// a.redo and formed after the loop with the operators, from global memory:
+// inlined into the loop, that body's registers would spill the fast one's.
+// 1920^2 Sedov: 0.38 ms, against 0.515 ms for one zone a thread with plain
+// loads and the division operator at 16 warps an SM; with this body 0.44 ms
+// at 12 warps and 0.52 ms at 16.  FP64 pipe 54% (its busy time alone is 0.18
+// ms), issue slots 50%.
+enum MeshKind { kGeneral, kQuads, kRect };
 
-// kRect: a rect mesh (a.rect_nzx > 0), point indices from the zone index.
-template <bool kQuads, bool kRect = false>
-__global__ void __launch_bounds__(kZoneThreadsZT, PNT_PASS_A_ZT_MIN_BLOCKS) pass_a_zt(DevArrays a, HydroConst c) {
+template <MeshKind kKind>
+__global__ void __launch_bounds__(32, 8) pass_a(DevArrays a, HydroConst c) {
+    extern __shared__ __align__(16) unsigned char smem_a[];
     pdl_wait();
     const Ctl* ctl = a.ctl;
     if (skip_cycle(ctl)) return;
-    const int64_t z = (int64_t)blockIdx.x * kZoneThreadsZT + threadIdx.x;
+    const int cur = ctl->cycle & 1;
+    const double dt = ctl->dt;
+    const int lane = threadIdx.x;
+    const int ntiles = (a.numz + zstage::kT - 1) / zstage::kT, step = (int)gridDim.x;
+    auto index = [&](int g) {
+        const int z = min(g * zstage::kT + lane, a.numz - 1);
+        if (kKind == kRect) return zstage::rect_idx(z, a.rect_nzx, 0, 0);
+        return zstage::load_idx(a, z, kKind == kQuads);
+    };
     double zdthyd = 1.e99;
     int bad = 0;
-    if (z < a.numz) {
-        const int cur = ctl->cycle & 1;
-        const double dt = ctl->dt;
-        if (kRect) {
-            const RectZoneIn in(a, cur, z);
-            pass_a_zone_thread<4>(a, c, in, dt, z, 4 * z, zdthyd, bad);
-        } else if (kQuads) {
-            pass_a_zone_thread<4>(a, c, cur, dt, z, 4 * z, zdthyd, bad);
-        } else {
-            const int n = a.znump[z];
-            const int64_t s0 = a.zfirst[z];
-            if (n == 4) pass_a_zone_thread<4>(a, c, cur, dt, z, s0, zdthyd, bad);
-            else pass_a_zone_thread<3>(a, c, cur, dt, z, s0, zdthyd, bad);
+    bool again = false;   // a zone of this warp is out of the straight-line form's range
+    int s = 0, g = (int)blockIdx.x;
+    zstage::Idx ix = index(min(g, ntiles - 1)), nx = ix;
+    if (g < ntiles) zstage::issue(a, cur, smem_a, ix);
+    tiles::commit();
+    if (g + step < ntiles) nx = index(g + step);
+    for (; g < ntiles; g += step) {
+        const int32_t z = ix.z, s0 = ix.s0, n = ix.n;
+        ix = nx;
+        if (g + step < ntiles) zstage::issue(a, cur, smem_a + (s ^ 1) * zstage::kBytes, ix);
+        tiles::commit();
+        if (g + 2 * step < ntiles) nx = index(g + 2 * step);
+        tiles::wait_groups<1>();   // this lane's copies of tile g have landed
+        const zstage::ZoneIn in{smem_a + s * zstage::kBytes, lane};
+        const bool own = g * zstage::kT + lane < a.numz;
+        bool ok = true;
+        if (own) {
+            double v = 1.e99;
+            int b = 0;
+            if (kKind != kGeneral || n == 4) ok = pass_a_zone_fast<4>(a, c, in, dt, z, s0, v, b);
+            else ok = pass_a_zone_fast<3>(a, c, in, dt, z, s0, v, b);
+            if (ok) {
+                zdthyd = dmin(zdthyd, v);
+                bad += b;
+            }
+        }
+        __syncwarp();
+        const unsigned m = __ballot_sync(kFull, !ok);
+        if (lane == 0) a.redo[g] = m;
+        again = again || m != 0;
+        s ^= 1;
+    }
+    if (again) {
+        __syncwarp();   // lane 0's notes
+        for (g = (int)blockIdx.x; g < ntiles; g += step) {
+            if (!((a.redo[g] >> lane) & 1)) continue;
+            const zstage::Idx r = index(g);
+            const GlobalZoneIn in{a, cur, r.z, r.s0};
+            double v = 1.e99;
+            if (kKind != kGeneral || r.n == 4) pass_a_zone_thread<4>(a, c, in, dt, r.z, r.s0, v, bad);
+            else pass_a_zone_thread<3>(a, c, in, dt, r.z, r.s0, v, bad);
+            zdthyd = dmin(zdthyd, v);
         }
     }
-    const int nbad = tiles::block_isum<kZoneThreadsZT>(bad);
-    block_to_cycle<true, kZoneThreadsZT>(a.cyc_red, zdthyd, nbad);
+    warp_to_cycle<true>(a.cyc_red, zdthyd, bad);
+}
+
+// Pass A of a small mesh: four lanes a zone, eight zones a warp, one warp a
+// CTA.
+template <MeshKind kKind>
+__global__ void __launch_bounds__(32) pass_a_small(DevArrays a, HydroConst c) {
+    pdl_wait();
+    const Ctl* ctl = a.ctl;
+    if (skip_cycle(ctl)) return;
+    const int cur = ctl->cycle & 1;
+    const double dt = ctl->dt;
+    const int lane = threadIdx.x;
+    const int zl = (int)blockIdx.x * 8 + (lane >> 2);
+    const bool live = zl < a.numz;
+    const int z = live ? zl : a.numz - 1;
+    const zstage::Idx ix =
+        kKind == kRect ? zstage::rect_idx(z, a.rect_nzx, 0, 0) : zstage::load_idx(a, z, kKind == kQuads);
+    double zdthyd = 1.e99;
+    int bad = 0;
+    const bool ok = pass_a_zone_lanes(a, c, cur, dt, z, ix.s0, ix.n, ix.p, live, zdthyd, bad);
+    const unsigned m = __ballot_sync(kFull, !ok) >> (lane & ~3);
+    if (m & 0xfu) {
+        zdthyd = 1.e99;
+        bad = 0;
+        if (live && (lane & 3) == 0) {
+            const GlobalZoneIn in{a, cur, z, ix.s0};
+            if (kKind != kGeneral || ix.n == 4) pass_a_zone_thread<4>(a, c, in, dt, z, ix.s0, zdthyd, bad);
+            else pass_a_zone_thread<3>(a, c, in, dt, z, ix.s0, zdthyd, bad);
+        }
+    }
+    __syncwarp();
+    warp_to_cycle<true>(a.cyc_red, zdthyd, bad);
 }
 
 template <bool kRect>
@@ -125,16 +193,29 @@ __global__ void piece_finish(DevArrays a, HydroConst c) {
     finish_cycle(ctl, c, r[0], -r[1], (int)r[2], (int)r[3]);
 }
 
+// Up to here a zone's four lanes beat its one thread: at 128^2 zones (14
+// warps an SM against 3.5) 10.6 against 11.0 us, at 48^2 8.5 against 10.5 us,
+// at 160^2 12.3 against 11.7 us (with the launch, about 3 us, in each; the
+// operators, a zone a thread, 13.9 us at 48^2).
+constexpr int kSmallZones = 16384;
+
+using PassA = void (*)(DevArrays, HydroConst);
+PassA pass_a_kernel(int32_t rect_nzx, bool quads) {
+    return rect_nzx > 0 ? pass_a<kRect> : (quads ? pass_a<kQuads> : pass_a<kGeneral>);
+}
+
 }  // namespace
 cudaError_t launch_cycle_fp64(const DevArrays& a, const HydroConst& c, cudaStream_t stream, cudaEvent_t* ev,
                               int phases) {
     const int pb = (int)((a.nump + kPointThreads - 1) / kPointThreads);
-    const int zba = (int)((a.numz + kZoneThreadsZT - 1) / kZoneThreadsZT);
     cudaError_t e = cudaSuccess;
     if (phases & kPhaseForces) {
         if (ev) cudaEventRecord(ev[0], stream);
-        e = launch_pdl(a.rect_nzx > 0 ? pass_a_zt<true, true> : (a.quads ? pass_a_zt<true> : pass_a_zt<false>), zba,
-                       kZoneThreadsZT, 0, stream, a, c);
+        if (a.numz <= kSmallZones)
+            e = launch_pdl(a.rect_nzx > 0 ? pass_a_small<kRect> : (a.quads ? pass_a_small<kQuads> : pass_a_small<kGeneral>),
+                           (a.numz + 7) / 8, 32, 0, stream, a, c);
+        else
+            e = launch_pdl(pass_a_kernel(a.rect_nzx, a.quads != 0), a.gridA, 32, zstage::kSmem, stream, a, c);
         if (ev) cudaEventRecord(ev[1], stream);
         if (ev) cudaEventRecord(ev[2], stream);   // no closure pass
     }
@@ -148,6 +229,19 @@ cudaError_t launch_cycle_fp64(const DevArrays& a, const HydroConst& c, cudaStrea
         if (ev) cudaEventRecord(ev[5], stream);   // no separate finalize step
     }
     return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+cudaError_t prepare_pass_a_fp64(int32_t rect_nzx, bool quads, int32_t numz, int nsm, int32_t* grid, int32_t* ntiles) {
+    *ntiles = (numz + zstage::kT - 1) / zstage::kT;
+    const auto k = pass_a_kernel(rect_nzx, quads);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, zstage::kSmem);
+    if (e != cudaSuccess) return e;
+    int occ = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 32, zstage::kSmem);
+    if (e != cudaSuccess) return e;
+    if (occ < 1) return cudaErrorInvalidConfiguration;
+    *grid = std::max(1, std::min(occ * nsm, *ntiles));
+    return cudaSuccess;
 }
 
 void launch_piece_pack(const DevArrays& a, const int32_t* send_side, int32_t nsend, unsigned char* send,

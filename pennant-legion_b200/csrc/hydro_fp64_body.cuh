@@ -11,7 +11,9 @@
 // serial CPU run of the reference bit for bit.
 #pragma once
 
+
 #include "hydro_dev.h"
+#include "ieee_div.cuh"
 
 #include <cuda_runtime.h>
 
@@ -140,6 +142,23 @@ __device__ __forceinline__ void block_to_cycle(long long* cyc_red, double v, int
     }
 }
 
+// The same for kernels whose CTAs are single warps: no barrier.
+template <bool kPassA>
+__device__ __forceinline__ void warp_to_cycle(long long* cyc_red, double v, int nbad) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const double w = __shfl_xor_sync(kFull, v, o);
+        v = kPassA ? dmin(v, w) : ((w > v) ? w : v);
+    }
+    nbad = (int)__reduce_add_sync(kFull, (unsigned)nbad);
+    if ((threadIdx.x & 31) == 0) {
+        if (v == v) {
+            if (kPassA) atomicMin(cyc_red, dkey(v));
+            else atomicMax(cyc_red + 1, dkey(v));
+        }
+        if (nbad)
+            atomicAdd(reinterpret_cast<unsigned long long*>(cyc_red + (kPassA ? 2 : 3)), (unsigned long long)nbad);
+    }
+}
 
 // ---------------------------------------------------------------------
 // Pass A, one corner of the QCS (QCS.cc:116-380), shared by the zone
@@ -401,12 +420,338 @@ __device__ __forceinline__ void pass_a_zone_thread(const DevArrays& a, const Hyd
     a.cforce[s0] = sub(ftot0, fprev);
 }
 
-// The same zone with its inputs gathered from global memory.
-template <int N>
-__device__ __forceinline__ void pass_a_zone_thread(const DevArrays& a, const HydroConst& c, int cur, double dt,
-                                                   int64_t z, int64_t s0, double& zdthyd, int& nbad) {
-    const GlobalZoneIn in{a, cur, z, s0};
-    pass_a_zone_thread<N>(a, c, in, dt, z, s0, zdthyd, nbad);
+// ---------------------------------------------------------------------
+// The same zone with its quotients and roots formed in straight-line code
+// (ieee_div.cuh): the same operations on the same operands in the same
+// order, so the same bits, for zones whose operands are all in range.
+// Returns false when one was not (an inverted zone, a run that blew up): the
+// zone's stores are then void and the caller forms it again with
+// pass_a_zone_thread.  Ahead of a shock the velocities die away over many
+// zones, through the smallest numbers there are, so where an operand can be
+// as small as they are it is not refused:
+//  - q and the velocity differences over the edges enter sums with, or are
+//    compared with, the sound speed, which is at least 1e-50: below that they
+//    need not be exact (quot_unchecked);
+//  - zkur adds du to the sound speed's term; where that is 2^-200 or more,
+//    a du below 2^-400 does not change it;
+//  - only the sign of the reference's cdiv is used: that of its dividend times
+//    that of its divisor, unless the quotient underflows, which it cannot
+//    over a divisor up to 1 (every edge below 1/2).
+// Other differences in form:
+//  - the corners' angles and weights are formed for all corners at once
+//    (their quotients interleave), and the side forces at the end from the
+//    half-step positions, which are live anyway.
+// The caller gives it 255 registers (8 warps an SM): at 168 it spills, which
+// costs more than the third warp a scheduler brings (zone_stage.cuh).
+// ---------------------------------------------------------------------
+template <int N, typename In>
+__device__ __forceinline__ bool pass_a_zone_fast(const DevArrays& a, const HydroConst& c, const In& in, double dt,
+                                                 int64_t z, int64_t s0, double& zdthyd, int& nbad) {
+    ieee::Guard g;
+    double2 xp[N], u0[N];
+    double mf[N];
+    const double dth = 0.5 * dt;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const double2 x0 = in.x0(k);
+        u0[k] = in.u0(k);
+        mf[k] = in.mf(k);
+        xp[k] = add(x0, smul(dth, u0[k]));   // advPosHalf
+    }
+    const double zm = in.zm(), zr = in.zr(), ze = in.ze(), zwrate = in.zwrate(), zvol0 = in.zvol();
+    const double rn = 1. / (double)N;
+    // calcCtrs, and the zone's velocity
+    double2 zxp = mk(__dadd_rn(0.0, xp[0].x * rn), __dadd_rn(0.0, xp[0].y * rn));
+    double2 zuc = mk(__dadd_rn(0.0, u0[0].x * rn), __dadd_rn(0.0, u0[0].y * rn));
+#pragma unroll
+    for (int k = 1; k < N; ++k) {
+        zxp = mk(zxp.x + xp[k].x * rn, zxp.y + xp[k].y * rn);
+        zuc = mk(zuc.x + u0[k].x * rn, zuc.y + u0[k].y * rn);
+    }
+    const double third = 1. / 3.;
+    const double fac = (N == 3 ? 3. : 4.);
+    double sa[N], elen[N], rinv[N];
+    double zareap = 0., zvolp = 0., zdl = 1.e99, dumax = 0.;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int nk = (k + 1 == N) ? 0 : k + 1;
+        const double2 dxs = sub(xp[nk], xp[k]);
+        sa[k] = 0.5 * cross(dxs, sub(zxp, xp[k]));
+        const double sv = third * sa[k] * (xp[k].x + xp[nk].x + zxp.x);
+        zareap = (k == 0) ? __dadd_rn(0.0, sa[k]) : zareap + sa[k];
+        zvolp = (k == 0) ? __dadd_rn(0.0, sv) : zvolp + sv;
+        nbad += (sv <= 0.) ? 1 : 0;
+        elen[k] = ieee::root(length2(dxs), g);
+        rinv[k] = ieee::rcp(elen[k], g);
+        zdl = dmin(zdl, ieee::quot(fac * sa[k], elen[k], rinv[k], g));
+        const double dux = dot(sub(u0[nk], u0[k]), dxs);
+        dumax = dmax(dumax, ieee::quot_unchecked(fabs(dux), elen[k], rinv[k]));
+    }
+    // PolyGas::calcStateHalf with calcRho
+    const double e = dmax(ze, 0.);
+    const double p = c.gm1 * zr * e;
+    const double pre = c.gm1 * e;
+    const double per = c.gm1 * zr;
+    const double q = ieee::quot_unchecked(per * p, zr * zr, ieee::rcp(zr * zr, g));
+    const double minv = ieee::rcp(zm, g);
+    const double csqd = dmax(c.ssmin2, pre + q);
+    const double zss = ieee::root(csqd, g);
+    const double dv = (zvolp - zvol0) * minv;
+    const double bulk = zr * csqd;
+    const double denom = 1. + 0.5 * per * dv;
+    const double src = zwrate * dth * minv;
+    const double zrp = ieee::quot(zm, zvolp, ieee::rcp(zvolp, g), g);
+    const double zp = p + ieee::quot1(per * src - zr * bulk * dv, denom, g);
+    a.zp[z] = zp;
+    const double zdu = c.q1 * zss + 2. * c.q2 * dumax;
+    const double cdu = dmax(zdu, dmax(zss, 1.e-99));
+    zdthyd = ieee::quot(zdl * c.cfl, cdu, ieee::rcp(cdu, g), g);
+    // calcCrnrMass and the TTS side pressures
+    double sstmp = dmax(zss, c.tts_ssmin);
+    sstmp = c.alfa * sstmp * sstmp;
+    double sdp[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int pk = (k == 0) ? N - 1 : k - 1;
+        a.cmass[s0 + k] = zrp * zareap * 0.5 * (mf[k] + mf[pk]);
+        const double vfacinv = ieee::quot(zareap, sa[k], ieee::rcp(sa[k], g), g);
+        const double srho = zrp * mf[k] * vfacinv;
+        sdp[k] = sstmp * (srho - zrp);
+    }
+    // every corner's angle and weight, and the sign of its velocity divergence
+    double cw[N], cc[N], sdiv[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int pk = (k == 0) ? N - 1 : k - 1;
+        const int nk = (k + 1 == N) ? 0 : k + 1;
+        const double2 x = xp[k], u = u0[k];
+        const double2 xq1 = smul(0.5, add(x, xp[nk])), xq3 = smul(0.5, add(xp[pk], x));
+        const double2 up1 = smul(0.5, add(u, u0[nk]));
+        const double2 up3 = smul(0.5, add(u0[pk], u));
+        const double2 d20 = sub(zxp, x), d31 = sub(xq3, xq1);
+        const double cvolume = 0.5 * cross(d20, d31);
+        const double minelen = dmin(elen[pk], elen[k]);
+        const double d12 = elen[pk] * elen[k];
+        const double cq = ieee::quot0(4. * dot(sub(xq3, x), sub(xq1, x)), d12, ieee::rcp(d12, g), g);
+        const double ccos = (minelen < 1.e-12) ? 0. : cq;
+        const double csin2 = 1.0 - ccos * ccos;
+        const bool flat = csin2 < 1.e-4;
+        const double cs = flat ? 1.0 : csin2;
+        cw[k] = flat ? 0. : ieee::quot(cvolume, cs, ieee::rcp(cs, g), g);
+        cc[k] = flat ? 0. : ccos;
+        const double num = cross(sub(zuc, u), d31) - cross(sub(up3, up1), d20);
+        g.divisor(2.0 * cvolume);
+        g.below(num);
+        sdiv[k] = (cvolume < 0.0) ? -num : num;
+    }
+    double emax = elen[0];
+#pragma unroll
+    for (int k = 1; k < N; ++k) emax = dmax(emax, elen[k]);
+    if (!(emax < 0.5)) {   // 2 cvolume may be over 1
+#pragma unroll
+        for (int k = 0; k < N; ++k) g.dividend(sdiv[k] == 0.0 ? 1.0 : sdiv[k]);
+    }
+    // the viscosity of each corner
+    const double ztmp1 = c.q1 * zss;
+    double crmu[N];
+    // no compression: zkur = sqrt(ztmp1^2) is a finite zkur >= +0, and (zkur
+    // zrp) 0 a zero with the sign of zrp
+    const bool heard = ztmp1 >= 0x1p-200;   // du below 2^-400 then leaves zkur at ztmp1
+    const bool still = fabs(ztmp1) < 1.e150 && fabs(zrp) < 1.e150 && c.q2 * 0.25 * c.gammap1 * 0.0 == 0.0 &&
+                       fabs(c.q2) < 0x1p100;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        crmu[k] = (sdiv[k] > 0.0) ? 0. : zrp * 0.0;
+        if (sdiv[k] < 0.0) {
+            const int pk = (k == 0) ? N - 1 : k - 1;
+            const int nk = (k + 1 == N) ? 0 : k + 1;
+            const double2 xq0 = xp[k], xq2 = zxp;
+            const double2 xq1 = smul(0.5, add(xq0, xp[nk])), xq3 = smul(0.5, add(xp[pk], xq0));
+            const double2 up0 = u0[k], up2 = zuc;
+            const double2 up1 = smul(0.5, add(up0, u0[nk]));
+            const double2 up3 = smul(0.5, add(u0[pk], up0));
+            const double cvolume = 0.5 * cross(sub(xq2, xq0), sub(xq3, xq1));
+            const double2 dxx1 = smul(0.5, sub(sub(add(xq1, xq2), xq0), xq3));
+            const double2 dxx2 = smul(0.5, sub(sub(add(xq2, xq3), xq0), xq1));
+            const double dx1 = ieee::root(length2(dxx1), g);
+            const double dx2 = ieee::root(length2(dxx2), g);
+            const double2 duav = smul(0.25, add(add(add(up0, up1), up2), up3));
+            const double test1 = fabs(dot(dxx1, duav) * dx2);
+            const double test2 = fabs(dot(dxx2, duav) * dx1);
+            const double num = (test1 > test2 ? dx1 : dx2);
+            const double den = (test1 > test2 ? dx2 : dx1);
+            const double r = ieee::quot(num, den, ieee::rcp(den, g), g);
+            const double evol = dmin(ieee::root(4.0 * cvolume * r, g), 2.0 * dmin(elen[pk], elen[k]));
+            const double dv1 = length2(sub(sub(add(up1, up2), up0), up3));
+            const double dv2 = length2(sub(sub(add(up2, up3), up0), up1));
+            const double dvm = dmax(dv1, dv2);
+            const double du = ieee::root((heard && dvm < 0x1p-800) ? 0x1p-800 : dvm, g);
+            const double ztmp2 = c.q2 * 0.25 * c.gammap1 * du;
+            const double zkur = ztmp2 + ieee::root(ztmp2 * ztmp2 + ztmp1 * ztmp1, g);
+            crmu[k] = zkur * zrp * evol;
+        }
+    }
+    // the sides: setForce, sftot, and the corner forces
+    double2 B0 = mk(0., 0.), Aprev = mk(0., 0.), ftot0 = mk(0., 0.), fprev = mk(0., 0.);
+    auto finish_side = [&](int j, double2 fs) {
+        const double2 ssurf = rotateCCW(sub(smul(0.5, add(xp[j], xp[(j + 1 == N) ? 0 : j + 1])), zxp));
+        const double2 sfpq = add(smul(-zp, ssurf), mk(fs.x * rinv[j], fs.y * rinv[j]));
+        const double2 ftot = add(sfpq, smul(-sdp[j], ssurf));
+        a.sftot[s0 + j] = sfpq;
+        if (j == 0) ftot0 = ftot;
+        else a.cforce[s0 + j] = sub(ftot, fprev);
+        fprev = ftot;
+    };
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int pk = (k == 0) ? N - 1 : k - 1;
+        const int nk = (k + 1 == N) ? 0 : k + 1;
+        const double2 u = u0[k];
+        const double2 t1 = smul(crmu[k], sub(u, u0[pk])), t2 = smul(crmu[k], sub(u0[nk], u));
+        const double2 cqe1 = mk(t1.x * rinv[pk], t1.y * rinv[pk]), cqe2 = mk(t2.x * rinv[k], t2.y * rinv[k]);
+        const double2 A = smul(cw[k], add(cqe2, smul(cc[k], cqe1)));
+        const double2 B = smul(cw[k], add(cqe1, smul(cc[k], cqe2)));
+        if (k == 0) B0 = B;
+        else finish_side(k - 1, add(Aprev, B));
+        Aprev = A;
+    }
+    finish_side(N - 1, add(Aprev, B0));
+    a.cforce[s0] = sub(ftot0, fprev);
+    return g.ok() && still;
+}
+
+// ---------------------------------------------------------------------
+// The straight-line zone over four lanes, lane k its side, corner and point
+// k (lane 3 idle in a triangle): for meshes of so few zones that a zone a
+// thread leaves most schedulers without a warp, where the time is one warp's
+// way through the code.  Zone quantities are formed in every lane, sums over
+// the sides in side order through shuffles, so the bits are those of
+// pass_a_zone_fast.  ix: the zone's points; a lane without a zone calls it
+// too (live = false, on any valid zone) and stores nothing.  Returns whether
+// the lane's operands were in range; the zone stands when all four lanes' were.
+// ---------------------------------------------------------------------
+__device__ __forceinline__ bool pass_a_zone_lanes(const DevArrays& a, const HydroConst& c, int cur, double dt,
+                                                  int32_t z, int32_t s0, int n, const int32_t* p, bool live,
+                                                  double& zdthyd, int& nbad) {
+    ieee::Guard g;
+    const int lane = threadIdx.x & 31, q = lane & 3, gl = lane & ~3;
+    const int k = q < n ? q : 0;                   // the lane's side (an idle lane repeats side 0)
+    const int ln = gl + ((k + 1 < n) ? k + 1 : 0), lp = gl + (k > 0 ? k - 1 : n - 1);
+    const bool mine = live && q < n;
+    const double dth = 0.5 * dt;
+    const int32_t pk = k == 0 ? p[0] : (k == 1 ? p[1] : (k == 2 ? p[2] : p[3]));
+    const double2 u = a.pu[cur][pk];
+    const double2 x = add(a.px[cur][pk], smul(dth, u));
+    const double mf = a.smf[s0 + k];
+    const double zm = a.zm[z], zr = a.zr[z], ze = a.ze[z], zwrate = a.zwrate[z], zvol0 = a.zvol[z];
+    const double2 xn = shfl2(x, ln), un = shfl2(u, ln), xv = shfl2(x, lp), uv = shfl2(u, lp);
+    const double mfv = shfl(mf, lp);
+    const double rn = n == 4 ? 1. / 4. : 1. / 3.;
+    const double2 zxp = zsum2(smul(rn, x), gl, n), zuc = zsum2(smul(rn, u), gl, n);
+    const double third = 1. / 3.;
+    const double fac = n == 4 ? 4. : 3.;
+    const double2 dxs = sub(xn, x);
+    const double sa = 0.5 * cross(dxs, sub(zxp, x));
+    const double sv = third * sa * (x.x + xn.x + zxp.x);
+    const double zareap = zsum(sa, gl, n), zvolp = zsum(sv, gl, n);
+    nbad += (mine && sv <= 0.) ? 1 : 0;
+    const double elen = ieee::root(length2(dxs), g);
+    const double rinv = ieee::rcp(elen, g);
+    const double elenv = shfl(elen, lp), rinvv = shfl(rinv, lp);
+    double zdl = dmin(1.e99, ieee::quot(fac * sa, elen, rinv, g));
+    double dumax = dmax(0., ieee::quot_unchecked(fabs(dot(sub(un, u), dxs)), elen, rinv));
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {   // an idle lane holds side 0's
+        zdl = dmin(zdl, __shfl_xor_sync(kFull, zdl, o));
+        dumax = dmax(dumax, __shfl_xor_sync(kFull, dumax, o));
+    }
+    // PolyGas::calcStateHalf with calcRho
+    const double e = dmax(ze, 0.);
+    const double pr = c.gm1 * zr * e;
+    const double pre = c.gm1 * e;
+    const double per = c.gm1 * zr;
+    const double qe = ieee::quot_unchecked(per * pr, zr * zr, ieee::rcp(zr * zr, g));
+    const double minv = ieee::rcp(zm, g);
+    const double csqd = dmax(c.ssmin2, pre + qe);
+    const double zss = ieee::root(csqd, g);
+    const double dv = (zvolp - zvol0) * minv;
+    const double bulk = zr * csqd;
+    const double denom = 1. + 0.5 * per * dv;
+    const double src = zwrate * dth * minv;
+    const double zrp = ieee::quot(zm, zvolp, ieee::rcp(zvolp, g), g);
+    const double zp = pr + ieee::quot1(per * src - zr * bulk * dv, denom, g);
+    const double zdu = c.q1 * zss + 2. * c.q2 * dumax;
+    const double cdu = dmax(zdu, dmax(zss, 1.e-99));
+    zdthyd = ieee::quot(zdl * c.cfl, cdu, ieee::rcp(cdu, g), g);
+    // calcCrnrMass and the TTS side pressure
+    double sstmp = dmax(zss, c.tts_ssmin);
+    sstmp = c.alfa * sstmp * sstmp;
+    const double cm = zrp * zareap * 0.5 * (mf + mfv);
+    const double vfacinv = ieee::quot(zareap, sa, ieee::rcp(sa, g), g);
+    const double srho = zrp * mf * vfacinv;
+    const double sdp = sstmp * (srho - zrp);
+    // the corner's angle and weight, and the sign of its velocity divergence
+    const double2 xq1 = smul(0.5, add(x, xn)), xq3 = smul(0.5, add(xv, x));
+    const double2 up1 = smul(0.5, add(u, un)), up3 = smul(0.5, add(uv, u));
+    const double2 d20 = sub(zxp, x), d31 = sub(xq3, xq1);
+    const double cvolume = 0.5 * cross(d20, d31);
+    const double minelen = dmin(elenv, elen);
+    const double d12 = elenv * elen;
+    const double cq = ieee::quot0(4. * dot(sub(xq3, x), sub(xq1, x)), d12, ieee::rcp(d12, g), g);
+    const double ccos = (minelen < 1.e-12) ? 0. : cq;
+    const double csin2 = 1.0 - ccos * ccos;
+    const bool flat = csin2 < 1.e-4;
+    const double cs = flat ? 1.0 : csin2;
+    const double cw = flat ? 0. : ieee::quot(cvolume, cs, ieee::rcp(cs, g), g);
+    const double cc = flat ? 0. : ccos;
+    const double num = cross(sub(zuc, u), d31) - cross(sub(up3, up1), d20);
+    g.divisor(2.0 * cvolume);
+    g.below(num);
+    g.dividend((fabs(cvolume) > 0.5 && num != 0.0) ? num : 1.0);
+    const double sdiv = (cvolume < 0.0) ? -num : num;
+    const double ztmp1 = c.q1 * zss;
+    const bool heard = ztmp1 >= 0x1p-200;   // du below 2^-400 then leaves zkur at ztmp1
+    const bool still = fabs(ztmp1) < 1.e150 && fabs(zrp) < 1.e150 && c.q2 * 0.25 * c.gammap1 * 0.0 == 0.0 &&
+                       fabs(c.q2) < 0x1p100;
+    double crmu = (sdiv > 0.0) ? 0. : zrp * 0.0;
+    if (sdiv < 0.0) {
+        const double2 dxx1 = smul(0.5, sub(sub(add(xq1, zxp), x), xq3));
+        const double2 dxx2 = smul(0.5, sub(sub(add(zxp, xq3), x), xq1));
+        const double dx1 = ieee::root(length2(dxx1), g);
+        const double dx2 = ieee::root(length2(dxx2), g);
+        const double2 duav = smul(0.25, add(add(add(u, up1), zuc), up3));
+        const double test1 = fabs(dot(dxx1, duav) * dx2);
+        const double test2 = fabs(dot(dxx2, duav) * dx1);
+        const double rnum = (test1 > test2 ? dx1 : dx2);
+        const double rden = (test1 > test2 ? dx2 : dx1);
+        const double r = ieee::quot(rnum, rden, ieee::rcp(rden, g), g);
+        const double evol = dmin(ieee::root(4.0 * cvolume * r, g), 2.0 * minelen);
+        const double dv1 = length2(sub(sub(add(up1, zuc), u), up3));
+        const double dv2 = length2(sub(sub(add(zuc, up3), u), up1));
+        const double dvm = dmax(dv1, dv2);
+        const double du = ieee::root((heard && dvm < 0x1p-800) ? 0x1p-800 : dvm, g);
+        const double ztmp2 = c.q2 * 0.25 * c.gammap1 * du;
+        const double zkur = ztmp2 + ieee::root(ztmp2 * ztmp2 + ztmp1 * ztmp1, g);
+        crmu = zkur * zrp * evol;
+    }
+    __syncwarp();
+    // setForce, sftot and the corner force of the lane's side
+    const double2 t1 = smul(crmu, sub(u, uv)), t2 = smul(crmu, sub(un, u));
+    const double2 cqe1 = mk(t1.x * rinvv, t1.y * rinvv), cqe2 = mk(t2.x * rinv, t2.y * rinv);
+    const double2 A = smul(cw, add(cqe2, smul(cc, cqe1)));
+    const double2 B = smul(cw, add(cqe1, smul(cc, cqe2)));
+    const double2 fs = add(A, shfl2(B, ln));
+    const double2 ssurf = rotateCCW(sub(xq1, zxp));
+    const double2 sfpq = add(smul(-zp, ssurf), mk(fs.x * rinv, fs.y * rinv));
+    const double2 ftot = add(sfpq, smul(-sdp, ssurf));
+    const double2 fv = shfl2(ftot, lp);
+    if (mine) {
+        a.cmass[s0 + k] = cm;
+        a.sftot[s0 + k] = sfpq;
+        a.cforce[s0 + k] = sub(ftot, fv);
+        if (k == 0) a.zp[z] = zp;
+    }
+    return g.ok() && still;
 }
 
 // ---------------------------------------------------------------------

@@ -32,6 +32,10 @@ __device__ __forceinline__ unsigned saddr(const void* p) { return (unsigned)__cv
 __device__ __forceinline__ void cp16(void* s, const void* g) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr(s)), "l"(g) : "memory");
 }
+// the same through L1, for lines that other lanes read too
+__device__ __forceinline__ void cp16a(void* s, const void* g) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(saddr(s)), "l"(g) : "memory");
+}
 __device__ __forceinline__ void cp8(void* s, const void* g) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(saddr(s)), "l"(g) : "memory");
 }
