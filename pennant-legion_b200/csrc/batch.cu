@@ -130,8 +130,10 @@ __global__ void __launch_bounds__(kBatchThreads) batch_point_pass(BatchDev b) {
         if (inst_skip(ctl)) continue;
         const HydroConst& c = b.consts[tile.inst];
         const int cur = ctl.cycle & 1;
-        for (int64_t p = (int64_t)tile.beg + threadIdx.x; p < tile.end; p += kBatchThreads)
-            pass_b_point(b.a, c, cur, ctl.dt, p);
+        for (int64_t pb = tile.beg; pb < tile.end; pb += kBatchThreads) {
+            const int64_t p = pb + threadIdx.x;
+            pass_b_point_csr<false>(b.a, c, cur, ctl.dt, p, p < tile.end);
+        }
     }
 }
 

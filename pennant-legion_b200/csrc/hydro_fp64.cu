@@ -146,14 +146,17 @@ __global__ void __launch_bounds__(32) pass_a_small(DevArrays a, HydroConst c) {
     warp_to_cycle<true>(a.cyc_red, zdthyd, bad);
 }
 
-template <bool kRect>
+template <bool kRectPoints>
 __global__ void __launch_bounds__(kPointThreads) pass_b(DevArrays a, HydroConst c) {
     pdl_wait();
     const Ctl* ctl = a.ctl;
     if (skip_cycle(ctl)) return;
     const int64_t p = (int64_t)blockIdx.x * kPointThreads + threadIdx.x;
-    if (p >= a.nump) return;
-    pass_b_point<kRect>(a, c, ctl->cycle & 1, ctl->dt, p);
+    if (kRectPoints) {
+        if (p < a.nump) pass_b_point_rect<false>(a, c, ctl->cycle & 1, ctl->dt, p);
+    } else {
+        pass_b_point_csr<false>(a, c, ctl->cycle & 1, ctl->dt, p, p < a.nump);
+    }
 }
 
 // Multi-piece runs: the corner values the neighbours need, and the end of

@@ -808,36 +808,108 @@ __device__ __forceinline__ int rect_point_corners(int32_t nzx, int32_t nzy, int6
     return n;
 }
 
-// kRect: a rect mesh (a.rect_nzx > 0), the point's corners from its index
-// instead of the CSR (the same sides in the same order).
-template <bool kRect = false>
-__device__ __forceinline__ void pass_b_point(const DevArrays& a, const HydroConst& c, int cur, double dt,
-                                             int64_t p) {
+// A point's corner mass and force, FP64 cycle (mixed = false) or widened
+// from FP32.
+template <bool kMixed>
+__device__ __forceinline__ void corner_values(const DevArrays& a, int64_t s, double& m, double2& f) {
+    if (kMixed) {
+        m = (double)a.cmass_f[s];
+        const float2 cf = a.cforce_f[s];
+        f = mk((double)cf.x, (double)cf.y);
+    } else {
+        m = a.cmass[s];
+        f = a.cforce[s];
+    }
+}
+
+// A point of a rect mesh (a.rect_nzx > 0): its corners from its index, in
+// ascending side order from zero (Hydro.cc:1100-1116, :1175-1192).
+template <bool kMixed>
+__device__ __forceinline__ void pass_b_point_rect(const DevArrays& a, const HydroConst& c, int cur, double dt,
+                                                  int64_t p) {
     const double2 x0 = a.px[cur][p];
     const double2 u0 = a.pu[cur][p];
-    // corner mass and force, ascending side order from zero (Hydro.cc:1100-1116, :1175-1192)
     double m = 0.;
     double2 f = mk(0., 0.);
-    if (kRect) {
-        int64_t sc[4];
-        const int n = rect_point_corners(a.rect_nzx, a.numz / a.rect_nzx, p, sc);
+    int64_t sc[4];
+    const int n = rect_point_corners(a.rect_nzx, a.numz / a.rect_nzx, p, sc);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (q < n) {
-                m = __dadd_rn(m, a.cmass[sc[q]]);
-                const double2 cf = a.cforce[sc[q]];
-                f = mk(__dadd_rn(f.x, cf.x), __dadd_rn(f.y, cf.y));
-            }
-        }
-    } else {
-        const int32_t o0 = a.poff[p], o1 = a.poff[p + 1];
-        for (int32_t i = o0; i < o1; ++i) {
-            const int32_t s = __ldg(a.pcorner + i);
-            m = __dadd_rn(m, a.cmass[s]);
-            const double2 cf = a.cforce[s];
+    for (int q = 0; q < 4; ++q) {
+        if (q < n) {
+            double cm;
+            double2 cf;
+            corner_values<kMixed>(a, sc[q], cm, cf);
+            m = __dadd_rn(m, cm);
             f = mk(__dadd_rn(f.x, cf.x), __dadd_rn(f.y, cf.y));
         }
     }
+    double2 x, u;
+    advance_point(c, dt, a.bcmask[p], m, f, x0, u0, x, u);
+    a.px[cur ^ 1][p] = x;
+    a.pu[cur ^ 1][p] = u;
+}
+
+// A point of any mesh through the point-to-corner CSR; called by whole warps
+// (live = false: no point).  A point of many corners, as the origin of a pie
+// mesh (as many as its triangles), would keep its thread for a gather latency
+// every few corners, 0.2 us a corner; so from 9 corners on (two of the
+// single thread's gather steps) the warp gathers them 32 at a time and three
+// lanes add mass and force in order from shared memory.  Pass B of a 313 x
+// 801 pie: 68 -> 18.6 us, of a 200 x 200 one 21.0 -> 10.6 us (3 us of each
+// the launch); what is left of the origin is the chain of its additions.
+constexpr int kManyCorners = 8;
+template <bool kMixed>
+__device__ __forceinline__ void pass_b_point_csr(const DevArrays& a, const HydroConst& c, int cur, double dt,
+                                                 int64_t p, bool live) {
+    int32_t o0 = 0, o1 = 0;
+    double2 x0 = mk(0., 0.), u0 = x0;
+    if (live) {
+        o0 = a.poff[p];
+        o1 = a.poff[p + 1];
+        x0 = a.px[cur][p];
+        u0 = a.pu[cur][p];
+    }
+    double m = 0.;
+    double2 f = mk(0., 0.);
+    const bool many = o1 - o0 > kManyCorners;
+    if (!many) {
+        for (int32_t i = o0; i < o1; ++i) {
+            double cm;
+            double2 cf;
+            corner_values<kMixed>(a, __ldg(a.pcorner + i), cm, cf);
+            m = __dadd_rn(m, cm);
+            f = mk(__dadd_rn(f.x, cf.x), __dadd_rn(f.y, cf.y));
+        }
+    }
+    const int lane = threadIdx.x & 31;
+    for (unsigned left = __ballot_sync(kFull, many); left; left &= left - 1) {
+        __shared__ double vals[kPointThreads / 32][3][32];   // mass, force x, force y of 32 corners
+        double(*v)[32] = vals[threadIdx.x >> 5];
+        const int who = __ffs(left) - 1;
+        const int32_t b = __shfl_sync(kFull, o0, who), e = __shfl_sync(kFull, o1, who);
+        const double* mine = v[min(lane, 2)];   // lanes 0, 1, 2 add one component each
+        double sum = 0., cm = 0.;
+        double2 cf = mk(0., 0.);
+        if (b + lane < e) corner_values<kMixed>(a, __ldg(a.pcorner + b + lane), cm, cf);
+        for (int32_t i = b; i < e; i += 32) {
+            v[0][lane] = cm;   // +0 past the last corner, which leaves the sums as they are
+            v[1][lane] = cf.x;
+            v[2][lane] = cf.y;
+            __syncwarp();
+            cm = 0.;
+            cf = mk(0., 0.);
+            if (i + 32 + lane < e) corner_values<kMixed>(a, __ldg(a.pcorner + i + 32 + lane), cm, cf);
+#pragma unroll
+            for (int q = 0; q < 32; ++q) sum = __dadd_rn(sum, mine[q]);
+            __syncwarp();
+        }
+        const double wm = shfl(sum, 0), wx = shfl(sum, 1), wy = shfl(sum, 2);
+        if (lane == who) {
+            m = wm;
+            f = mk(wx, wy);
+        }
+    }
+    if (!live) return;
     double2 x, u;
     advance_point(c, dt, a.bcmask[p], m, f, x0, u0, x, u);
     a.px[cur ^ 1][p] = x;

@@ -883,49 +883,17 @@ __global__ void
 // ---------------------------------------------------------------------
 // Pass B, mixed: FP32 corner inputs summed in FP64
 // ---------------------------------------------------------------------
-// kRect: a rect mesh, the point's corners from its index
-// (fp64::rect_point_corners: the CSR's sides in the CSR's order).
-template <bool kRect = false>
-__device__ __forceinline__ void pass_b_mixed_point(const DevArrays& a, const HydroConst& c, int cur, double dt,
-                                                   int64_t p) {
-    const double2 x0 = a.px[cur][p];
-    const double2 u0 = a.pu[cur][p];
-    double m = 0.;
-    double2 f = mk(0., 0.);
-    if (kRect) {
-        int64_t sc[4];
-        const int n = fp64::rect_point_corners(a.rect_nzx, a.numz / a.rect_nzx, p, sc);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (q < n) {
-                m = __dadd_rn(m, (double)a.cmass_f[sc[q]]);
-                const float2 cf = a.cforce_f[sc[q]];
-                f = mk(__dadd_rn(f.x, (double)cf.x), __dadd_rn(f.y, (double)cf.y));
-            }
-        }
-    } else {
-        const int32_t o0 = a.poff[p], o1 = a.poff[p + 1];
-        for (int32_t i = o0; i < o1; ++i) {
-            const int32_t s = __ldg(a.pcorner + i);
-            m = __dadd_rn(m, (double)a.cmass_f[s]);
-            const float2 cf = a.cforce_f[s];
-            f = mk(__dadd_rn(f.x, (double)cf.x), __dadd_rn(f.y, (double)cf.y));
-        }
-    }
-    double2 x, u;
-    fp64::advance_point(c, dt, a.bcmask[p], m, f, x0, u0, x, u);
-    a.px[cur ^ 1][p] = x;
-    a.pu[cur ^ 1][p] = u;
-}
-
 template <bool kRect>
 __global__ void __launch_bounds__(kPointThreads) pass_b_mixed(DevArrays a, HydroConst c) {
     pdl_wait();
     const Ctl* ctl = a.ctl;
     if (skip_cycle(ctl)) return;
     const int64_t p = (int64_t)blockIdx.x * kPointThreads + threadIdx.x;
-    if (p >= a.nump) return;
-    pass_b_mixed_point<kRect>(a, c, ctl->cycle & 1, ctl->dt, p);
+    if (kRect) {
+        if (p < a.nump) fp64::pass_b_point_rect<true>(a, c, ctl->cycle & 1, ctl->dt, p);
+    } else {
+        fp64::pass_b_point_csr<true>(a, c, ctl->cycle & 1, ctl->dt, p, p < a.nump);
+    }
 }
 
 // ---------------------------------------------------------------------
@@ -977,8 +945,10 @@ __global__ void __launch_bounds__(kBatchThreads) batch_point_pass_mixed(BatchDev
         if (inst_skip(ctl)) continue;
         const HydroConst& c = b.consts[tile.inst];
         const int cur = ctl.cycle & 1;
-        for (int64_t p = (int64_t)tile.beg + threadIdx.x; p < tile.end; p += kBatchThreads)
-            pass_b_mixed_point(b.a, c, cur, ctl.dt, p);
+        for (int64_t pb = tile.beg; pb < tile.end; pb += kBatchThreads) {
+            const int64_t p = pb + threadIdx.x;
+            fp64::pass_b_point_csr<true>(b.a, c, cur, ctl.dt, p, p < tile.end);
+        }
     }
 }
 
