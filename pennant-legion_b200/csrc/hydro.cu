@@ -309,8 +309,8 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
             e = prepare_pass_a_fp64(a.rect_nzx, a.quads != 0, a.numz, nsm, &a.gridA, &ntiles);
             if (e != cudaSuccess) return fail(PNT_ERR_CUDA, "pass A setup: %s", cudaGetErrorString(e));
             if (pnt_status st = h->alloc(&a.redo, (size_t)ntiles)) return st;
-        } else if (a.rect_nzx > 0) {
-            e = prepare_pass_a_rows_mixed(p.precision == PNT_PREC_LEARNED, a.rect_nzx, a.numz, nsm, &a.gridA);
+        } else {
+            e = prepare_pass_a_mixed(p.precision == PNT_PREC_LEARNED, a.rect_nzx, a.quads != 0, a.numz, nsm, &a.gridA);
             if (e != cudaSuccess) return fail(PNT_ERR_CUDA, "pass A setup: %s", cudaGetErrorString(e));
         }
     }

@@ -98,7 +98,7 @@ struct DevArrays {
     int32_t closure_grid;   // CTAs of the persistent closure pass
     uint32_t* redo;         // FP64 pass A: the zones of each warp tile that are formed again (hydro_fp64.cu)
     int32_t gridC;          // CTAs of the persistent pass C (pass_c_staged.cuh)
-    int32_t gridA;          // CTAs of the persistent pass A (FP64; mixed and learned on rect meshes)
+    int32_t gridA;          // CTAs of the persistent pass A
     // multi-piece runs: pass C's last CTA writes this piece's [dtnew,
     // -dvovmax, inverted sides in A, in C] here instead of ending the cycle
     // (nullptr for a single piece)
@@ -183,14 +183,12 @@ cudaError_t prepare_learned_kernels();
 // write a.gridC partials.
 cudaError_t prepare_pass_c(bool mixed, bool quads, int32_t rect_nzx, int32_t numz, int nsm, int32_t* grid);
 void launch_pass_c(const DevArrays& a, const HydroConst& c, bool mixed, cudaStream_t stream);
-// Pass A of the FP64 cycle (hydro_fp64.cu): the kernel's shared-memory limit
-// on the current device, its persistent grid, and the warp tiles a.redo holds
-// a word for.
+// Pass A of the FP64 cycle (hydro_fp64.cu) and of the mixed or learned cycle
+// (hydro_mixed.cu): raises the kernel's shared-memory limit on the current
+// device and returns its persistent grid (and the tiles a.redo holds a word
+// for).
 cudaError_t prepare_pass_a_fp64(int32_t rect_nzx, bool quads, int32_t numz, int nsm, int32_t* grid, int32_t* ntiles);
-// The row-tile pass A of the mixed or learned cycle (hydro_mixed.cu): raises
-// the kernel's shared-memory limit on the current device and returns its
-// persistent grid.
-cudaError_t prepare_pass_a_rows_mixed(bool learned, int32_t rect_nzx, int32_t numz, int nsm, int32_t* grid);
+cudaError_t prepare_pass_a_mixed(bool learned, int32_t rect_nzx, bool quads, int32_t numz, int nsm, int32_t* grid);
 
 // Device state of a pnt_hydro for the closure harvest (closure.cu).
 struct HydroAccess {

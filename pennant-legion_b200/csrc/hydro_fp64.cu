@@ -39,16 +39,18 @@ namespace {
 
 using namespace fp64;
 
-// Pass A: one warp a CTA, 8 an SM, each walking tiles of 32 zones (tiles
-// blockIdx.x, blockIdx.x + gridDim.x, ...) through its two stages
-// (zone_stage.cuh).  Zones that the straight-line body refuses are noted in
+// Pass A: one warp a CTA, 8 an SM, each walking tiles of 32 zones through its
+// two stages (zone_stage.cuh).  Zones that the straight-line body refuses are noted in
 // a.redo and formed after the loop with the operators, from global memory:
 // inlined into the loop, that body's registers would spill the fast one's.
 // 1920^2 Sedov: 0.38 ms, against 0.515 ms for one zone a thread with plain
 // loads and the division operator at 16 warps an SM; with this body 0.44 ms
 // at 12 warps and 0.52 ms at 16.  FP64 pipe 54% (its busy time alone is 0.18
 // ms), issue slots 50%.
-enum MeshKind { kGeneral, kQuads, kRect };
+using zstage::MeshKind;
+using zstage::kGeneral;
+using zstage::kQuads;
+using zstage::kRect;
 
 template <MeshKind kKind>
 __global__ void __launch_bounds__(32, 8) pass_a(DevArrays a, HydroConst c) {
@@ -59,29 +61,12 @@ __global__ void __launch_bounds__(32, 8) pass_a(DevArrays a, HydroConst c) {
     const int cur = ctl->cycle & 1;
     const double dt = ctl->dt;
     const int lane = threadIdx.x;
-    const int ntiles = (a.numz + zstage::kT - 1) / zstage::kT, step = (int)gridDim.x;
-    auto index = [&](int g) {
-        const int z = min(g * zstage::kT + lane, a.numz - 1);
-        if (kKind == kRect) return zstage::rect_idx(z, a.rect_nzx, 0, 0);
-        return zstage::load_idx(a, z, kKind == kQuads);
-    };
+    const int w = (int)blockIdx.x, nw = (int)gridDim.x;
     double zdthyd = 1.e99;
     int bad = 0;
     bool again = false;   // a zone of this warp is out of the straight-line form's range
-    int s = 0, g = (int)blockIdx.x;
-    zstage::Idx ix = index(min(g, ntiles - 1)), nx = ix;
-    if (g < ntiles) zstage::issue(a, cur, smem_a, ix);
-    tiles::commit();
-    if (g + step < ntiles) nx = index(g + step);
-    for (; g < ntiles; g += step) {
-        const int32_t z = ix.z, s0 = ix.s0, n = ix.n;
-        ix = nx;
-        if (g + step < ntiles) zstage::issue(a, cur, smem_a + (s ^ 1) * zstage::kBytes, ix);
-        tiles::commit();
-        if (g + 2 * step < ntiles) nx = index(g + 2 * step);
-        tiles::wait_groups<1>();   // this lane's copies of tile g have landed
-        const zstage::ZoneIn in{smem_a + s * zstage::kBytes, lane};
-        const bool own = g * zstage::kT + lane < a.numz;
+    zstage::for_tiles<kKind>(a, cur, smem_a, w, nw,
+                             [&](const zstage::ZoneIn& in, int g, int32_t z, int32_t s0, int n, bool own) {
         bool ok = true;
         if (own) {
             double v = 1.e99;
@@ -97,17 +82,18 @@ __global__ void __launch_bounds__(32, 8) pass_a(DevArrays a, HydroConst c) {
         const unsigned m = __ballot_sync(kFull, !ok);
         if (lane == 0) a.redo[g] = m;
         again = again || m != 0;
-        s ^= 1;
-    }
+    });
     if (again) {
         __syncwarp();   // lane 0's notes
-        for (g = (int)blockIdx.x; g < ntiles; g += step) {
+        const int ntiles = (a.numz + zstage::kT - 1) / zstage::kT;
+        for (int g = w; g < ntiles; g += nw) {
             if (!((a.redo[g] >> lane) & 1)) continue;
-            const zstage::Idx r = index(g);
-            const GlobalZoneIn in{a, cur, r.z, r.s0};
+            const int32_t z = g * zstage::kT + lane;
+            const int32_t s0 = kKind == kGeneral ? a.zfirst[z] : 4 * z;
+            const GlobalZoneIn in{a, cur, z, s0};
             double v = 1.e99;
-            if (kKind != kGeneral || r.n == 4) pass_a_zone_thread<4>(a, c, in, dt, r.z, r.s0, v, bad);
-            else pass_a_zone_thread<3>(a, c, in, dt, r.z, r.s0, v, bad);
+            if (kKind != kGeneral || a.znump[z] == 4) pass_a_zone_thread<4>(a, c, in, dt, z, s0, v, bad);
+            else pass_a_zone_thread<3>(a, c, in, dt, z, s0, v, bad);
             zdthyd = dmin(zdthyd, v);
         }
     }
@@ -236,15 +222,7 @@ cudaError_t launch_cycle_fp64(const DevArrays& a, const HydroConst& c, cudaStrea
 
 cudaError_t prepare_pass_a_fp64(int32_t rect_nzx, bool quads, int32_t numz, int nsm, int32_t* grid, int32_t* ntiles) {
     *ntiles = (numz + zstage::kT - 1) / zstage::kT;
-    const auto k = pass_a_kernel(rect_nzx, quads);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, zstage::kSmem);
-    if (e != cudaSuccess) return e;
-    int occ = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 32, zstage::kSmem);
-    if (e != cudaSuccess) return e;
-    if (occ < 1) return cudaErrorInvalidConfiguration;
-    *grid = std::max(1, std::min(occ * nsm, *ntiles));
-    return cudaSuccess;
+    return zstage::prepare(pass_a_kernel(rect_nzx, quads), rect_nzx, numz, nsm, grid);
 }
 
 void launch_piece_pack(const DevArrays& a, const int32_t* send_side, int32_t nsend, unsigned char* send,

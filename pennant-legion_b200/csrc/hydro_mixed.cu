@@ -21,9 +21,7 @@
 // around each zone, and calcWork needs that cancellation), and sfp + sfq is
 // handed to calcWork in FP64; the corner mass and corner force handed to the
 // point pass are stored in FP32 (4 + 8 B per side instead of 24 B).  Pass A
-// runs one thread per zone (128 registers, 4 blocks of 128 per SM): with the
-// divisions and square roots in FP32 it is 40% faster than four lanes per
-// zone.  The learned cycle (precision learned) is this cycle with the QCS
+// runs one thread per zone, 8 warps an SM.  The learned cycle (precision learned) is this cycle with the QCS
 // corner forces of compressing corners moved to the closure pass.
 // Compiled with fast math; the accuracy of this path is stated as its L1
 // error against the FP64 run (tests/test_gpu_mixed.py).
@@ -31,10 +29,11 @@
 #include "hydro_fp64_body.cuh"
 #include "batch_dev.h"
 #include "hydro_dev.h"
-#include "row_tiles.cuh"
-#include "zone_tiles.cuh"
+#include "zone_stage.cuh"
 
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 namespace pnt {
 namespace {
@@ -187,6 +186,14 @@ struct SideSpill {
     __device__ __forceinline__ float2& sft(int k) const { return sft_[k * stride + t]; }
 };
 
+// The same held in registers, for a kernel that has them.
+struct SideRegs {
+    mutable double2 p[4];
+    mutable float2 t[4];
+    __device__ __forceinline__ double2& sfp(int k) const { return p[k]; }
+    __device__ __forceinline__ float2& sft(int k) const { return t[k]; }
+};
+
 // Where the learned cycle's pass A records a zone for the closure: record
 // i at base + (i & mask) * kZoneRecF4, i from an atomic counter (global or
 // shared memory).
@@ -200,10 +207,10 @@ struct RecSink {
 // compression, in the dead zone, in an acute zone (learned cycle).
 // in: the zone's inputs (fp64::GlobalZoneIn, or a row tile's shared-memory
 // stage); sink: where a zone with deferred corners is recorded (learned).
-template <int N, bool kLearned, typename In>
+template <int N, bool kLearned, typename In, typename Park>
 __device__ __forceinline__ void pass_a_mixed_zone(const DevArrays& a, const HydroConst& c, const In& in, int cur,
                                                   double dt, int64_t z, int64_t s0, double& zdthyd, int& nbad,
-                                                  int* cnt, const SideSpill& sp, const RecSink& sink = RecSink{}) {
+                                                  int* cnt, const Park& sp, const RecSink& sink = RecSink{}) {
     double2 xp[N];
     float2 uf[N];
     double mf[N];
@@ -247,17 +254,27 @@ __device__ __forceinline__ void pass_a_mixed_zone(const DevArrays& a, const Hydr
     // QCS, the corner mass, the Courant dt), so they are formed in FP32.
     // q = per p / zr^2 is written gm1 pre (the same quantity, no division).
     const double e = dmax(ze, 0.);
-    const double p = c.gm1 * zr * e;
     const double pre = c.gm1 * e;
     const double per = c.gm1 * zr;
     const double q = c.gm1 * pre;
-    const double minv = 1. / zm;
     const double csqd = dmax(c.ssmin2, pre + q);
-    const double dv = (zvolp - zvol0) * minv;
     const double bulk = zr * csqd;
-    const double denom = 1. + 0.5 * per * dv;
-    const double src = zwrate * dth * minv;
-    const double zp = p + (per * src - zr * bulk * dv) / denom;
+    ieee::Guard g;
+    auto eos_num = [&](double minv, double dv) {
+        const double src = zwrate * dth * minv;
+        return per * src - zr * bulk * dv;
+    };
+    double minv = ieee::rcp(zm, g);
+    double dv = (zvolp - zvol0) * minv;
+    double denom = 1. + 0.5 * per * dv;
+    double dp = ieee::quot1(eos_num(minv, dv), denom, g);
+    if (!g.ok()) {   // out of the straight-line form's range (ieee_div.cuh): the operators
+        minv = 1. / zm;
+        dv = (zvolp - zvol0) * minv;
+        denom = 1. + 0.5 * per * dv;
+        dp = eos_num(minv, dv) / denom;
+    }
+    const double zp = __fma_rn(c.gm1 * zr, e, dp);
     const float zssf = sqrtf((float)csqd);
     const float zrpf = (float)zm / (float)zvolp;
     {
@@ -305,7 +322,7 @@ __device__ __forceinline__ void pass_a_mixed_zone(const DevArrays& a, const Hydr
         for (int k = 0; k < N; ++k) {
             const int nk = (k + 1 == N) ? 0 : k + 1;
             const double2 ex64 = smul(0.5, add(xp[k], xp[nk]));
-            sp.sfp(k) = smul(-zp, mk(-(ex64.y - zxp.y), ex64.x - zxp.x));
+            sp.sfp(k) = mk(__dmul_rn(-zp, -(ex64.y - zxp.y)), __dmul_rn(-zp, ex64.x - zxp.x));
             const float2 ssurf = fk(-(ex[k].y - zc.y), ex[k].x - zc.x);
             const float srho = zrpf * (float)mf[k] * (zareapf / (float)sa[k]);
             sp.sft(k) = fmul(-(sstmp * (srho - zrpf)), ssurf);
@@ -795,89 +812,67 @@ __device__ __forceinline__ void closure_add_counts(const DevArrays& a, const uns
         atomicAdd(a.closure_counts + kClassZones * 64 + (blockIdx.x & 63), (unsigned long long)zones);
 }
 
-// Pass A over row tiles of a rect mesh (row_tiles.cuh): the same zone body
-// reading its inputs from the tile's shared-memory stage, persistent CTAs,
-// two stages, 96-zone tiles and CTAs of 96 threads, 4 CTAs per SM (168
-// registers).  At 1920^2 Sedov the learned pass A takes 0.231 ms, against
-// 0.236 ms with 128-zone tiles (3 CTAs per SM), 0.236 ms with 64-zone tiles
-// (6 CTAs), 0.247-0.254 ms with 64-zone tiles held to 144 or 128 registers
-// (7 or 8 CTAs, spills) and 0.258 ms for the gathering kernel; three stages
-// were slower (fewer resident CTAs).
-#ifndef PNT_ROWS_A_STAGES
-#define PNT_ROWS_A_STAGES 2
-#endif
-#ifndef PNT_ROWS_A_T
-#define PNT_ROWS_A_T 96
-#endif
-#ifndef PNT_ROWS_A_MIN_BLOCKS
-#define PNT_ROWS_A_MIN_BLOCKS 4
-#endif
-constexpr int kRowsAStages = PNT_ROWS_A_STAGES;
-constexpr int kRowsAT = PNT_ROWS_A_T;   // zones a tile, threads a CTA
-using AStage = rows::PassAStage<kRowsAT>;
-constexpr int kRowsASmem = kRowsAStages * AStage::kBytes;
-
-template <bool kLearned>
-__global__ void
-#ifdef PNT_ROWS_A_MAXREG
-    __maxnreg__(PNT_ROWS_A_MAXREG)
-#else
-    __launch_bounds__(kRowsAT, PNT_ROWS_A_MIN_BLOCKS)
-#endif
-    pass_a_mixed_rows(DevArrays a, HydroConst c) {
-    extern __shared__ __align__(128) unsigned char smem_a[];
-    __shared__ __align__(8) uint64_t bars[kRowsAStages];
-    __shared__ double2 s_sfp[4 * kRowsAT];
-    __shared__ float2 s_sft[4 * kRowsAT];
+// Pass A: one warp a CTA, 8 an SM, each walking tiles of 32 zones through
+// two stages of its own (zone_stage.cuh).  1920^2 Sedov, mixed / learned:
+// 0.251 / 0.218 ms, against 0.291 / 0.258 ms for CTAs of 96 zones with a
+// barrier a tile (12 warps an SM, 168 registers); with 12 or 16 warps this way
+// 0.34-0.40 ms (spills, and stages that leave 30 KB of L1).  The EOS's two
+// divisions in straight-line code gave 0.010 ms of it.
+template <zstage::MeshKind kKind, bool kLearned>
+__global__ void __launch_bounds__(32, 8) pass_a_mixed(DevArrays a, HydroConst c) {
+    extern __shared__ __align__(16) unsigned char smem_a[];
     pdl_wait();
     const Ctl* ctl = a.ctl;
     if (skip_cycle(ctl)) return;
     const int cur = ctl->cycle & 1;
     const double dt = ctl->dt;
-    const int32_t nzx = a.rect_nzx;
-    const int64_t npx = (int64_t)nzx + 1;
-    const int64_t ntiles = rows::num_tiles<kRowsAT>(nzx, a.numz);
-    const int t = threadIdx.x;
-    const SideSpill sp{s_sfp, s_sft, t, kRowsAT};
+    const int lane = threadIdx.x;
+    // parked: 2880x288 Leblanc 0.0512 (shared memory) against 0.0530 ms; in
+    // the learned cycle, whose corner loop is short, 0.0517 against 0.0508 ms
+    using Park = std::conditional_t<kLearned, SideRegs, SideSpill>;
+    Park sp{};
+    if constexpr (!kLearned) {
+        __shared__ double2 s_sfp[4 * 32];
+        __shared__ float2 s_sft[4 * 32];
+        sp = SideSpill{s_sfp, s_sft, lane, 32};
+    }
+    const RecSink sink{a.closure_nrec, reinterpret_cast<float4*>(a.closure_rec), 0x7fffffff};
     double zdthyd = 1.e99;
     int bad = 0;
     int cnt[3] = {0, 0, 0};
-    const RecSink sink{a.closure_nrec, reinterpret_cast<float4*>(a.closure_rec), 0x7fffffff};
-    auto bytes = [&](int64_t g) { return AStage::bytes(rows::tile_of<kRowsAT>(g, nzx)); };
-    auto issue = [&](unsigned char* st, int64_t g, uint32_t bar) {
-        AStage::issue(st, a, cur, rows::tile_of<kRowsAT>(g, nzx), npx, bar);
-    };
-    auto compute = [&](const unsigned char* st, int64_t g) {
-        const rows::Tile tl = rows::tile_of<kRowsAT>(g, nzx);
-        if (t >= tl.nt) return;
-        const rows::RowZoneIn<kRowsAT> in{st, t, (int)(tl.z0 & 1)};
-        const int64_t z = tl.z0 + t;
+    zstage::for_tiles<kKind>(a, cur, smem_a, (int)blockIdx.x, (int)gridDim.x,
+                             [&](const zstage::ZoneIn& in, int, int32_t z, int32_t s0, int n, bool own) {
+        if (!own) return;
         double v = 1.e99;
         int zc[3] = {0, 0, 0};   // the zone's own corner classes (an acute zone overwrites them)
-        pass_a_mixed_zone<4, kLearned>(a, c, in, cur, dt, z, 4 * z, v, bad, zc, sp, sink);
+        if (kKind != zstage::kGeneral || n == 4)
+            pass_a_mixed_zone<4, kLearned>(a, c, in, cur, dt, z, s0, v, bad, zc, sp, sink);
+        else
+            pass_a_mixed_zone<3, kLearned>(a, c, in, cur, dt, z, s0, v, bad, zc, sp, sink);
         zdthyd = dmin(zdthyd, v);
 #pragma unroll
         for (int q = 0; q < 3; ++q) cnt[q] += zc[q];
-    };
-    if (!rows::for_tiles<kRowsAStages, AStage::kBytes>(ntiles, smem_a, bars, bytes, issue, compute) && t == 0)
-        atomicOr(reinterpret_cast<unsigned long long*>(a.cyc_red + 4), 1ull);
-    __shared__ unsigned wcount[kLearned ? kRowsAT / 32 : 1][3];
-    if constexpr (kLearned) {
-        for (int q = 0; q < 3; ++q) {
-            const unsigned tt = __reduce_add_sync(kFull, (unsigned)cnt[q]);
-            if ((threadIdx.x & 31) == 0) wcount[threadIdx.x >> 5][q] = tt;
-        }
-    }
-    const int nbad = tiles::block_isum<kRowsAT>(bad);   // its barrier also orders wcount
+    });
     if constexpr (kLearned) {
         constexpr int kCounted[3] = {kClassZero, kClassDead, kClassAcute};
-        if (threadIdx.x < 3) {
-            unsigned tt = 0;
-            for (int w = 0; w < kRowsAT / 32; ++w) tt += wcount[w][threadIdx.x];
-            if (tt) atomicAdd(a.closure_counts + kCounted[threadIdx.x] * 64 + (blockIdx.x & 63), (unsigned long long)tt);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const unsigned t = __reduce_add_sync(kFull, (unsigned)cnt[q]);
+            if (lane == 0 && t)
+                atomicAdd(a.closure_counts + kCounted[q] * 64 + (blockIdx.x & 63), (unsigned long long)t);
         }
     }
-    fp64::block_to_cycle<true, kRowsAT>(a.cyc_red, zdthyd, nbad);
+    fp64::warp_to_cycle<true>(a.cyc_red, zdthyd, bad);
+}
+
+using PassA = void (*)(DevArrays, HydroConst);
+template <bool kLearned>
+PassA pass_a_kernel(int32_t rect_nzx, bool quads) {
+    return rect_nzx > 0 ? pass_a_mixed<zstage::kRect, kLearned>
+                        : (quads ? pass_a_mixed<zstage::kQuads, kLearned> : pass_a_mixed<zstage::kGeneral, kLearned>);
+}
+PassA pass_a_kernel(bool learned, int32_t rect_nzx, bool quads) {
+    return learned ? pass_a_kernel<true>(rect_nzx, quads) : pass_a_kernel<false>(rect_nzx, quads);
 }
 
 // ---------------------------------------------------------------------
@@ -989,21 +984,13 @@ namespace {
 cudaError_t launch_cycle_mixed_impl(const DevArrays& a, const HydroConst& c, cudaStream_t stream, cudaEvent_t* ev,
                                     bool learned, int phases) {
     const int pb = (int)((a.nump + kPointThreads - 1) / kPointThreads);
-    const int zba = (int)((a.numz + kZoneThreadsZT - 1) / kZoneThreadsZT);
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t r) {
         if (e == cudaSuccess) e = r;
     };
     if (phases & kPhaseForces) {
         if (ev) cudaEventRecord(ev[0], stream);
-        if (a.rect_nzx > 0) {
-            chk(launch_pdl(learned ? pass_a_mixed_rows<true> : pass_a_mixed_rows<false>, a.gridA, kRowsAT, kRowsASmem,
-                           stream, a, c));
-        } else {
-            auto k = learned ? (a.quads ? pass_a_mixed_zt<true, true> : pass_a_mixed_zt<false, true>)
-                             : (a.quads ? pass_a_mixed_zt<true, false> : pass_a_mixed_zt<false, false>);
-            chk(launch_pdl(k, zba, kZoneThreadsZT, 0, stream, a, c));
-        }
+        chk(launch_pdl(pass_a_kernel(learned, a.rect_nzx, a.quads != 0), a.gridA, 32, zstage::kSmem, stream, a, c));
         if (ev) cudaEventRecord(ev[1], stream);
         if (learned) chk(launch_pdl(closure_pass, a.closure_grid, kCpThreads, kCpSmemBytes, stream, a, c));
         if (ev) cudaEventRecord(ev[2], stream);
@@ -1031,10 +1018,8 @@ cudaError_t launch_cycle_learned(const DevArrays& a, const HydroConst& c, cudaSt
     return launch_cycle_mixed_impl(a, c, stream, ev, true, phases);
 }
 
-cudaError_t prepare_pass_a_rows_mixed(bool learned, int32_t rect_nzx, int32_t numz, int nsm, int32_t* grid) {
-    const int64_t nt = rows::num_tiles<kRowsAT>(rect_nzx, numz);
-    return learned ? rows::prepare(pass_a_mixed_rows<true>, kRowsAT, kRowsASmem, nt, nsm, grid)
-                   : rows::prepare(pass_a_mixed_rows<false>, kRowsAT, kRowsASmem, nt, nsm, grid);
+cudaError_t prepare_pass_a_mixed(bool learned, int32_t rect_nzx, bool quads, int32_t numz, int nsm, int32_t* grid) {
+    return zstage::prepare(pass_a_kernel(learned, rect_nzx, quads), rect_nzx, numz, nsm, grid);
 }
 
 void launch_batch_pass_a_mixed(const BatchDev& b, bool all_quads, cudaStream_t stream) {

@@ -159,79 +159,5 @@ __device__ __forceinline__ bool for_tiles(int64_t ntiles, unsigned char* smem, u
     return ok;
 }
 
-// ---------------------------------------------------------------------
-// Pass A's stage: position and velocity (current buffer) of the tile's
-// bottom and top point rows, the side mass fractions of its 4T sides and
-// five zone fields, T (even) zones a tile.
-// ---------------------------------------------------------------------
-template <int T>
-struct PassAStage {
-    static constexpr int kRB = (T + 1) * 16;        // one point row of a double2 field
-    static constexpr int kOffMf = 4 * kRB;          // [X0 b,t][U0 b,t], then smf
-    static constexpr int kOffZs = kOffMf + 32 * T;  // zm, zr, ze, zwrate, zvol: T + 2 each
-    static constexpr int kZB = (T + 2) * 8;
-    static constexpr int kBytes = kOffZs + 5 * kZB;
-    static_assert(T % 2 == 0 && kBytes % 16 == 0, "16-byte aligned stages");
-
-    __device__ static uint32_t bytes(const Tile& tl) {
-        return (uint32_t)(4 * (tl.nt + 1) * 16 + 32 * tl.nt + 5 * zone_run(tl).count * 8);
-    }
-    __device__ static void issue(unsigned char* st, const DevArrays& a, int cur, const Tile& tl, int64_t npx,
-                                 uint32_t bar) {
-        const ZoneRun zr = zone_run(tl);
-        const uint32_t rb = (uint32_t)(tl.nt + 1) * 16;
-        bulk_g2s(st, a.px[cur] + tl.pb, rb, bar);
-        bulk_g2s(st + kRB, a.px[cur] + tl.pb + npx, rb, bar);
-        bulk_g2s(st + 2 * kRB, a.pu[cur] + tl.pb, rb, bar);
-        bulk_g2s(st + 3 * kRB, a.pu[cur] + tl.pb + npx, rb, bar);
-        bulk_g2s(st + kOffMf, a.smf + 4 * tl.z0, (uint32_t)(32 * tl.nt), bar);
-        const double* zf[5] = {a.zm, a.zr, a.ze, a.zwrate, a.zvol};
-#pragma unroll
-        for (int f = 0; f < 5; ++f) bulk_g2s(st + kOffZs + f * kZB, zf[f] + zr.zs, (uint32_t)(zr.count * 8), bar);
-    }
-};
-
-// Zone t of a pass A stage, read as fp64::GlobalZoneIn reads global memory:
-// side k of a rect zone starts at point (i, j), (i+1, j), (i+1, j+1),
-// (i, j+1) for k = 0..3.
-template <int T>
-struct RowZoneIn {
-    const unsigned char* st;
-    int t, shift;
-    __device__ __forceinline__ const double2* pt(int f, int k) const {
-        return reinterpret_cast<const double2*>(st + (2 * f + (k >= 2 ? 1 : 0)) * PassAStage<T>::kRB) + t +
-               ((k == 1 || k == 2) ? 1 : 0);
-    }
-    __device__ __forceinline__ double2 x0(int k) const { return *pt(0, k); }
-    __device__ __forceinline__ double2 u0(int k) const { return *pt(1, k); }
-    __device__ __forceinline__ double mf(int k) const {
-        return reinterpret_cast<const double*>(st + PassAStage<T>::kOffMf)[4 * t + k];
-    }
-    __device__ __forceinline__ double zs(int f) const {
-        return reinterpret_cast<const double*>(st + PassAStage<T>::kOffZs + f * PassAStage<T>::kZB)[shift + t];
-    }
-    __device__ __forceinline__ double zm() const { return zs(0); }
-    __device__ __forceinline__ double zr() const { return zs(1); }
-    __device__ __forceinline__ double ze() const { return zs(2); }
-    __device__ __forceinline__ double zwrate() const { return zs(3); }
-    __device__ __forceinline__ double zvol() const { return zs(4); }
-};
-
-// Persistent grid of a row-tile kernel: resident CTAs per SM x nsm, at
-// most one per tile.
-template <typename K>
-inline cudaError_t prepare(K k, int threads, int smem_bytes, int64_t ntiles, int nsm, int32_t* grid) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e != cudaSuccess) return e;
-    int occ = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, threads, smem_bytes);
-    if (e != cudaSuccess) return e;
-    if (occ < 1) return cudaErrorInvalidConfiguration;
-    int64_t g = (int64_t)occ * nsm;
-    if (g > ntiles) g = ntiles;
-    *grid = (int32_t)(g < 1 ? 1 : g);
-    return cudaSuccess;
-}
-
 }  // namespace rows
 }  // namespace pnt

@@ -97,5 +97,74 @@ struct ZoneIn {
     __device__ __forceinline__ double zvol() const { return zs(4); }
 };
 
+// How a mesh's zones and sides are numbered: any way, quads at sides 4z ..
+// 4z + 3, or as the rect generator does (row_tiles.cuh).
+enum MeshKind { kGeneral, kQuads, kRect };
+
+// The zones of one mesh, one warp's share: tiles w, w + nw, ...  compute(in,
+// g, z, s0, n, own) is called by whole warps for each tile g: the lane's zone
+// z with sides s0 .. s0 + n - 1 (own = false past the last zone).
+template <MeshKind kKind, typename Compute>
+__device__ __forceinline__ void for_tiles(const DevArrays& a, int cur, unsigned char* smem, int w, int nw,
+                                          Compute&& compute) {
+    const int lane = threadIdx.x & 31;
+    const int ntiles = (a.numz + kT - 1) / kT;
+    auto index = [&](int g) {
+        const int z = min(g * kT + lane, a.numz - 1);
+        if (kKind == kRect) return rect_idx(z, a.rect_nzx, 0, 0);
+        return load_idx(a, z, kKind == kQuads);
+    };
+    if (w >= ntiles) return;
+    Idx ix = index(w), nx = ix;
+    issue(a, cur, smem, ix);
+    tiles::commit();
+    if (w + nw < ntiles) nx = index(w + nw);
+    int s = 0;
+    for (int g = w; g < ntiles; g += nw) {
+        const int32_t z = ix.z, s0 = ix.s0, n = kKind == kGeneral ? ix.n : 4;
+        ix = nx;
+        if (g + nw < ntiles) issue(a, cur, smem + (s ^ 1) * kBytes, ix);
+        tiles::commit();
+        if (g + 2 * nw < ntiles) nx = index(g + 2 * nw);
+        tiles::wait_groups<1>();   // this lane's copies of tile g have landed
+        compute(ZoneIn{smem + s * kBytes, lane}, g, z, s0, n, g * kT + lane < a.numz);
+        __syncwarp();
+        s ^= 1;
+    }
+}
+
+// Raises the shared-memory limit of a kernel of one-warp CTAs and returns its
+// persistent grid: resident CTAs per SM x nsm, at most one per tile.  Where
+// nw tiles are (nearly) whole rows of a rect mesh, a warp would keep to the
+// same columns, and the warps whose columns a shock crosses would have all
+// the compressing zones (1024^2 Sedov: 37 rows a round, 5.9 of 8 warps active
+// on average); the grid is then cut by up to 2% so that the columns move on.
+template <typename K>
+inline cudaError_t prepare(K k, int32_t rect_nzx, int32_t numz, int nsm, int32_t* grid) {
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (e != cudaSuccess) return e;
+    int occ = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 32, kSmem);
+    if (e != cudaSuccess) return e;
+    if (occ < 1) return cudaErrorInvalidConfiguration;
+    const int tiles = (numz + kT - 1) / kT;
+    int nw = occ * nsm < tiles ? occ * nsm : tiles;
+    if (rect_nzx > 0 && tiles > nw) {
+        // how far a round moves a warp along the rows, and over the mesh
+        auto drift = [&](int n) {
+            const double f = (double)n * kT / rect_nzx, d = f - (double)(long long)f;
+            return (d < 0.5 ? d : 1. - d) * tiles / n;
+        };
+        if (drift(nw) < 1.) {
+            int best = nw;
+            for (int n = nw; n >= nw - nw / 50 && n > 0; --n)
+                if (drift(n) > drift(best)) best = n;
+            nw = best;
+        }
+    }
+    *grid = nw;
+    return cudaSuccess;
+}
+
 }  // namespace zstage
 }  // namespace pnt
