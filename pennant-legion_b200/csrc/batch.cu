@@ -7,17 +7,22 @@
 // uneven size share the GPU without a launch per mesh, and instances that
 // are done are skipped tile by tile.  The per-zone and per-point
 // arithmetic is the FP64 body shared with the single-mesh kernels
-// (pass A: pass_a_zone_thread of hydro_fp64_body.cuh, one thread per zone;
-// pass C: the staged corrector of pass_c_staged.cuh), so every instance is
-// bit-identical to its own single-mesh run; tiles only change which CTA
-// does the work.  Pass A runs one CTA per zone tile; passes B and C are
-// persistent.  The batch cycle is captured in a CUDA graph.  The tile size
+// (pass A: pass_a_zone_fast of hydro_fp64_body.cuh through the warp stages
+// of zone_stage.cuh; pass C: the staged corrector of pass_c_staged.cuh), so
+// every instance is bit-identical to its own single-mesh run; tiles only
+// change which CTA does the work.  The batch cycle is captured in a CUDA
+// graph, its kernels launched with programmatic dependent launch.  12
+// instances of 36^2 to 453^2 zones: FP64 cycle 0.171 -> 0.137 ms with this
+// pass A (0.8 of the gain), rect instances' corners from the point index and
+// the dependent launches; mixed, 52^2 to 352^2: 0.090 -> 0.083 ms.  The tile
+// size
 // (passes A and C) and the point pass's CTAs per SM are picked by
 // pnt_batch_tune, which times candidate shapes on the run's own cycles (the
 // results do not depend on the shape).
 //
 // Compiled with -fmad=false (FP64 parity).
 #include "batch_dev.h"
+#include "batch_tiles.cuh"
 #include "hydro_fp64_body.cuh"
 #include "pass_c_staged.cuh"
 #include "pnt_internal.h"
@@ -36,47 +41,58 @@ namespace {
 
 using namespace fp64;
 
-// Pass A: one CTA per tile (no persistent loop: its state would cost the
-// zone body registers), one thread per zone (pass_a_zone_thread), 128 zones
-// per step through the tile; one partial per tile.
-// kAllQuads: every instance's zones are quads at sides 4z..4z+3, so only
-// the 4-sided body is compiled (fewer registers than the general form).
+// Pass A: the single-mesh kernel's zone loop (hydro_fp64.cu) over the warp
+// tiles of the batch.  kAllQuads: every instance's zones are quads at sides
+// 4z..4z+3, so only the 4-sided body is compiled.
 template <bool kAllQuads>
-__global__ void __launch_bounds__(kBatchZT, 3) batch_pass_a(BatchDev b) {
-    {
-        const int t = blockIdx.x;
-        if (t >= b.nztiles) return;   // no tiles left: the grid is one idle CTA
-        const Tile tile = b.ztiles[t];
-        const Ctl& ctl = b.ctls[tile.inst];
-        if (inst_skip(ctl)) return;   // uniform over the CTA
-        const HydroConst& c = b.consts[tile.inst];
-        const int cur = ctl.cycle & 1;
-        const double dt = ctl.dt;
-        double fold = 1.e99;
-        int nbad = 0;
-        for (int zb = tile.beg; zb < tile.end; zb += kBatchZT) {
-            const int64_t z = (int64_t)zb + threadIdx.x;
-            if (z >= tile.end) continue;
+__global__ void __launch_bounds__(32, 8) batch_pass_a(BatchDev b) {
+    extern __shared__ __align__(16) unsigned char smem_a[];
+    pdl_wait();
+    const int lane = threadIdx.x, w = (int)blockIdx.x, nw = (int)gridDim.x;
+    btiles::InstFold fold;
+    bool again = false;   // a zone of this warp is out of the straight-line form's range
+    btiles::for_tiles<kAllQuads>(b, smem_a, w, nw,
+                                 [&](const zstage::ZoneIn& in, int g, int inst, const HydroConst& c, double dt, int32_t z,
+                                     int32_t s0, int n, bool own) {
+        fold.at(b, inst);
+        bool ok = true;
+        if (own) {
             double v = 1.e99;
-            if (tile.nzx > 0) {   // a rect instance: point indices from the zone index
-                const RectZoneIn in(b.a, cur, z, tile.nzx, z - tile.zo, tile.po);
-                pass_a_zone_thread<4>(b.a, c, in, dt, z, 4 * z, v, nbad);
-            } else if (kAllQuads || tile.quads) {
-                const GlobalZoneIn in{b.a, cur, z, 4 * z};
-                pass_a_zone_thread<4>(b.a, c, in, dt, z, 4 * z, v, nbad);
-            } else {
-                const int n = b.a.znump[z];
-                const int64_t s0 = b.a.zfirst[z];
-                const GlobalZoneIn in{b.a, cur, z, s0};
-                if (n == 4) pass_a_zone_thread<4>(b.a, c, in, dt, z, s0, v, nbad);
-                else pass_a_zone_thread<3>(b.a, c, in, dt, z, s0, v, nbad);
+            int bad = 0;
+            if (kAllQuads || n == 4) ok = pass_a_zone_fast<4>(b.a, c, in, dt, z, s0, v, bad);
+            else ok = pass_a_zone_fast<3>(b.a, c, in, dt, z, s0, v, bad);
+            if (ok) {
+                fold.v = dmin(fold.v, v);
+                fold.bad += bad;
             }
-            fold = dmin(fold, v);
         }
-        nbad = tiles::block_isum<kBatchZT>(nbad);
-        block_fold<true, kBatchZT>(fold, b.a.part_dtnew + t);
-        if (threadIdx.x == 0) b.a.part_badA[t] = nbad;
+        __syncwarp();
+        const unsigned m = __ballot_sync(kFull, !ok);
+        if (lane == 0) b.a.redo[g] = m;
+        again = again || m != 0;
+    });
+    if (again) {
+        __syncwarp();   // lane 0's notes
+        for (int g = w; g < b.nztiles * b.subs; g += nw) {
+            const btiles::WarpTile t = btiles::warp_tile<kAllQuads>(b, g, btiles::load_entry(b, g));
+            if (!t.any()) continue;
+            const unsigned m = b.a.redo[g];
+            if (!m) continue;
+            fold.at(b, t.inst);
+            if ((m >> lane) & 1) {
+                const Ctl& ctl = b.ctls[t.inst];
+                const GlobalZoneIn in{b.a, ctl.cycle & 1, t.ix.z, t.ix.s0};
+                double v = 1.e99;
+                if (kAllQuads || t.ix.n == 4)
+                    pass_a_zone_thread<4>(b.a, b.consts[t.inst], in, ctl.dt, t.ix.z, t.ix.s0, v, fold.bad);
+                else
+                    pass_a_zone_thread<3>(b.a, b.consts[t.inst], in, ctl.dt, t.ix.z, t.ix.s0, v, fold.bad);
+                fold.v = dmin(fold.v, v);
+            }
+            __syncwarp();
+        }
     }
+    fold.flush(b);
 }
 
 // Pass C: the staged corrector of pass_c_staged.cuh, one stage, its
@@ -87,6 +103,7 @@ __global__ void __launch_bounds__(kBatchZT, 3) batch_pass_a(BatchDev b) {
 template <bool kAllQuads, bool kMixed>
 __global__ void __launch_bounds__(stagedc::kTile) batch_pass_c(BatchDev b) {
     extern __shared__ __align__(16) unsigned char smem_c[];
+    pdl_wait();
     const int th = threadIdx.x;
     for (int t = blockIdx.x; t < b.nztiles; t += gridDim.x) {
         const Tile tile = b.ztiles[t];
@@ -124,6 +141,7 @@ __global__ void __launch_bounds__(stagedc::kTile) batch_pass_c(BatchDev b) {
 }
 
 __global__ void __launch_bounds__(kBatchThreads) batch_point_pass(BatchDev b) {
+    pdl_wait();
     for (int t = blockIdx.x; t < b.nptiles; t += gridDim.x) {
         const Tile tile = b.ptiles[t];
         const Ctl& ctl = b.ctls[tile.inst];
@@ -132,35 +150,42 @@ __global__ void __launch_bounds__(kBatchThreads) batch_point_pass(BatchDev b) {
         const int cur = ctl.cycle & 1;
         for (int64_t pb = tile.beg; pb < tile.end; pb += kBatchThreads) {
             const int64_t p = pb + threadIdx.x;
-            pass_b_point_csr<false>(b.a, c, cur, ctl.dt, p, p < tile.end);
+            if (tile.nzx > 0) {
+                if (p < tile.end)
+                    pass_b_point_rect<false>(b.a, c, cur, ctl.dt, p, tile.nzx, tile.nzy, tile.po, 4 * (int64_t)tile.zo);
+            } else {
+                pass_b_point_csr<false>(b.a, c, cur, ctl.dt, p, p < tile.end);
+            }
         }
     }
 }
 
 // One warp per instance: reduce its tiles' partials and end its cycle.
 __global__ void __launch_bounds__(kBatchThreads) batch_finalize(BatchDev b) {
+    pdl_wait();
     const int inst = (int)((blockIdx.x * (int64_t)kBatchThreads + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (inst >= b.ninst) return;   // whole warps leave together
     Ctl* ctl = b.ctls + inst;
     if (inst_skip(*ctl)) return;
-    double dtn = 1.e99, dvm = 1.e-99;
-    int badA = 0, badC = 0;
+    double dvm = 1.e-99;
+    int badC = 0;
     for (int t = b.inst_tbeg[inst] + lane; t < b.inst_tbeg[inst + 1]; t += 32) {
-        dtn = dmin(dtn, b.a.part_dtnew[t]);
         const double v = b.a.part_dvov[t];
         dvm = (v > dvm) ? v : dvm;
-        badA += b.a.part_badA[t];
         badC += b.a.part_badC[t];
     }
     for (int o = 16; o > 0; o >>= 1) {
-        dtn = dmin(dtn, __shfl_xor_sync(kFull, dtn, o));
         const double w = __shfl_xor_sync(kFull, dvm, o);
         dvm = (w > dvm) ? w : dvm;
-        badA += __shfl_xor_sync(kFull, badA, o);
         badC += __shfl_xor_sync(kFull, badC, o);
     }
-    if (lane == 0) finish_cycle(ctl, b.consts[inst], dtn, dvm, badA, badC);
+    if (lane == 0) {
+        long long* r = b.inst_red + 2 * inst;
+        finish_cycle(ctl, b.consts[inst], dkey_value(r[0]), dvm, (int)r[1], badC);
+        r[0] = dkey(1.e99);
+        r[1] = 0;
+    }
 }
 
 // Count of instances still running, for the host's stop test.
@@ -218,11 +243,13 @@ struct pnt_batch {
     Shape shape{256, 3};
     int nsm = 148;
     int grid_c = 148;                            // resident pass C CTAs (occupancy x SMs)
+    int32_t grid_a = 148;                        // resident pass A warps
     // device tile lists (rebuilt when the shape changes)
     Tile* ztiles = nullptr;
     Tile* ptiles = nullptr;
     int32_t* inst_tbeg = nullptr;
     void* parts = nullptr;
+    uint32_t* redo = nullptr;
     cudaGraphExec_t graph = nullptr;
     int graph_cycles = 8;
     int32_t live = 0;                            // instances in the current work lists
@@ -238,6 +265,7 @@ struct pnt_batch {
         if (ptiles) cudaFree(ptiles);
         if (inst_tbeg) cudaFree(inst_tbeg);
         if (parts) cudaFree(parts);
+        if (redo) cudaFree(redo);
         if (ctl_host) cudaFreeHost(ctl_host);
         if (running_host) cudaFreeHost(running_host);
         if (stream) cudaStreamDestroy(stream);
@@ -258,6 +286,8 @@ struct pnt_batch {
         return PNT_OK;
     }
 
+    int32_t rect_nzy(int i) const { return rect_nzx[i] > 0 ? nz[i] / rect_nzx[i] : 0; }
+
     // Work lists for a tile shape over the instances still running (ctl_host
     // must be current); partial arrays sized to the zone tiles.  Finished
     // instances get no tiles, so the persistent passes do not walk them.
@@ -274,9 +304,10 @@ struct pnt_batch {
             listed[i] = 1;
             for (int64_t z = 0; z < nz[i]; z += sh.zones_per_tile)
                 zt.push_back({i, (int32_t)(zoff[i] + z), (int32_t)(zoff[i] + std::min<int64_t>(nz[i], z + sh.zones_per_tile)),
-                              quads[i], rect_nzx[i], (int32_t)zoff[i], (int32_t)poff[i], 0});
+                              quads[i], rect_nzx[i], (int32_t)zoff[i], (int32_t)poff[i], rect_nzy(i)});
             for (int64_t p = 0; p < np[i]; p += ppt)
-                pt.push_back({i, (int32_t)(poff[i] + p), (int32_t)(poff[i] + std::min<int64_t>(np[i], p + ppt)), quads[i]});
+                pt.push_back({i, (int32_t)(poff[i] + p), (int32_t)(poff[i] + std::min<int64_t>(np[i], p + ppt)),
+                              quads[i], rect_nzx[i], (int32_t)zoff[i], (int32_t)poff[i], rect_nzy(i)});
         }
         tb[ninst] = (int32_t)zt.size();
         live = nlive;
@@ -286,12 +317,15 @@ struct pnt_batch {
         if (ptiles) cudaFree(ptiles);
         if (inst_tbeg) cudaFree(inst_tbeg);
         if (parts) cudaFree(parts);
-        ztiles = nullptr; ptiles = nullptr; inst_tbeg = nullptr; parts = nullptr;
+        if (redo) cudaFree(redo);
+        ztiles = nullptr; ptiles = nullptr; inst_tbeg = nullptr; parts = nullptr; redo = nullptr;
         const size_t nzt = zt.size();
         CUDA_TRY(cudaMalloc(&ztiles, std::max<size_t>(nzt, 1) * sizeof(Tile)));
         CUDA_TRY(cudaMalloc(&ptiles, std::max<size_t>(pt.size(), 1) * sizeof(Tile)));
         CUDA_TRY(cudaMalloc(&inst_tbeg, tb.size() * sizeof(int32_t)));
-        CUDA_TRY(cudaMalloc(&parts, std::max<size_t>(nzt, 1) * (2 * sizeof(double) + 2 * sizeof(int32_t))));
+        const int subs = (sh.zones_per_tile + zstage::kT - 1) / zstage::kT;
+        CUDA_TRY(cudaMalloc(&parts, std::max<size_t>(nzt, 1) * (sizeof(double) + sizeof(int32_t))));
+        CUDA_TRY(cudaMalloc(&redo, std::max<size_t>(nzt, 1) * subs * sizeof(uint32_t)));
         if (nzt) CUDA_TRY(cudaMemcpy(ztiles, zt.data(), nzt * sizeof(Tile), cudaMemcpyHostToDevice));
         if (!pt.empty()) CUDA_TRY(cudaMemcpy(ptiles, pt.data(), pt.size() * sizeof(Tile), cudaMemcpyHostToDevice));
         CUDA_TRY(cudaMemcpy(inst_tbeg, tb.data(), tb.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
@@ -300,11 +334,10 @@ struct pnt_batch {
         b.nztiles = (int32_t)nzt;
         b.nptiles = (int32_t)pt.size();
         b.inst_tbeg = inst_tbeg;
-        b.a.part_dtnew = static_cast<double*>(parts);
-        b.a.part_dvov = b.a.part_dtnew + nzt;
-        b.a.part_badA = reinterpret_cast<int32_t*>(b.a.part_dvov + nzt);
-        b.a.part_badC = b.a.part_badA + nzt;
-        b.a.npartA = b.a.npartC = (int32_t)nzt;
+        b.subs = subs;
+        b.a.part_dvov = static_cast<double*>(parts);
+        b.a.part_badC = reinterpret_cast<int32_t*>(b.a.part_dvov + nzt);
+        b.a.redo = redo;
         shape = sh;
         return PNT_OK;
     }
@@ -312,27 +345,26 @@ struct pnt_batch {
     cudaError_t launch_cycle(cudaEvent_t* ev = nullptr) {
         const int grid_p = std::max(1, std::min(b.nptiles, nsm * shape.ctas_per_sm));
         const int grid_f = (ninst * 32 + kBatchThreads - 1) / kBatchThreads;
-        if (ev) cudaEventRecord(ev[0], stream);
-        if (mixed) launch_batch_pass_a_mixed(b, all_quads, stream);
-        else if (all_quads) batch_pass_a<true><<<std::max(1, b.nztiles), kBatchZT, 0, stream>>>(b);
-        else batch_pass_a<false><<<std::max(1, b.nztiles), kBatchZT, 0, stream>>>(b);
-        if (ev) cudaEventRecord(ev[1], stream);
-        if (mixed) launch_batch_point_pass_mixed(b, grid_p, stream);
-        else batch_point_pass<<<grid_p, kBatchThreads, 0, stream>>>(b);
-        if (ev) cudaEventRecord(ev[2], stream);
         const int gc = std::max(1, std::min(b.nztiles, grid_c));
-        const size_t smc = stagedc::kSmemBytes;
-        if (mixed) {
-            if (all_quads) batch_pass_c<true, true><<<gc, stagedc::kTile, smc, stream>>>(b);
-            else batch_pass_c<false, true><<<gc, stagedc::kTile, smc, stream>>>(b);
-        } else {
-            if (all_quads) batch_pass_c<true, false><<<gc, stagedc::kTile, smc, stream>>>(b);
-            else batch_pass_c<false, false><<<gc, stagedc::kTile, smc, stream>>>(b);
-        }
+        const int ga = std::max(1, std::min(b.nztiles * b.subs, (int)grid_a));
+        cudaError_t e = cudaSuccess;
+        auto chk = [&](cudaError_t r) {
+            if (e == cudaSuccess) e = r;
+        };
+        if (ev) cudaEventRecord(ev[0], stream);
+        if (mixed) chk(launch_batch_pass_a_mixed(b, all_quads, stream));
+        else chk(launch_pdl(all_quads ? batch_pass_a<true> : batch_pass_a<false>, ga, 32, zstage::kSmem, stream, b));
+        if (ev) cudaEventRecord(ev[1], stream);
+        if (mixed) chk(launch_batch_point_pass_mixed(b, grid_p, stream));
+        else chk(launch_pdl(batch_point_pass, grid_p, kBatchThreads, 0, stream, b));
+        if (ev) cudaEventRecord(ev[2], stream);
+        auto kc = mixed ? (all_quads ? batch_pass_c<true, true> : batch_pass_c<false, true>)
+                        : (all_quads ? batch_pass_c<true, false> : batch_pass_c<false, false>);
+        chk(launch_pdl(kc, gc, stagedc::kTile, stagedc::kSmemBytes, stream, b));
         if (ev) cudaEventRecord(ev[3], stream);
-        batch_finalize<<<grid_f, kBatchThreads, 0, stream>>>(b);
+        chk(launch_pdl(batch_finalize, grid_f, kBatchThreads, 0, stream, b));
         if (ev) cudaEventRecord(ev[4], stream);
-        return cudaGetLastError();
+        return e != cudaSuccess ? e : cudaGetLastError();
     }
 
     pnt_status ensure_graph() {
@@ -574,7 +606,7 @@ pnt_status pnt_batch_create(const pnt_mesh* const* meshes, const pnt_params* par
             (st = bt->alloc(&a.zr, NZ)) || (st = bt->alloc(&a.ze, NZ)) || (st = bt->alloc(&a.zetot, NZ)) ||
             (st = bt->alloc(&a.zwrate, NZ)) || (st = bt->alloc(&a.zvol, NZ)) || (st = bt->alloc(&a.zp, NZ)) ||
             (st = bt->alloc(&a.cmass, NS)) || (st = bt->alloc(&a.cforce, NS)) || (st = bt->alloc(&a.sftot, NS)) ||
-            (st = bt->alloc(&d_consts, n)) || (st = bt->alloc(&d_ctls, n)) || (st = bt->alloc(&bt->running_dev, 1))) {
+            (st = bt->alloc(&d_consts, n)) || (st = bt->alloc(&d_ctls, n)) || (st = bt->alloc(&bt->b.inst_red, 2 * n)) || (st = bt->alloc(&bt->running_dev, 1))) {
             delete bt;
             return st;
         }
@@ -608,6 +640,12 @@ pnt_status pnt_batch_create(const pnt_mesh* const* meshes, const pnt_params* par
                 (e = up(d_ctls, ctls.data(), sizeof(Ctl) * n)))
                 ;
         }
+        if (e == cudaSuccess) {
+            std::vector<long long> red(2 * (size_t)n, 0);   // minimum from 1e99 (the key of a positive double is its bits)
+            const double lo = 1.e99;
+            for (int i = 0; i < n; ++i) std::memcpy(&red[2 * (size_t)i], &lo, 8);
+            e = up(bt->b.inst_red, red.data(), red.size() * 8);
+        }
         if (e == cudaSuccess) e = cudaMemset(a.zp, 0, NZ * 8);
         if (e == cudaSuccess) e = cudaMemset(d_mask + NP, 0, 4);   // pass C copies 32-bit mask words
         if (e == cudaSuccess) {
@@ -623,6 +661,9 @@ pnt_status pnt_batch_create(const pnt_mesh* const* meshes, const pnt_params* par
                     stagedc::kSmemBytes);
             if (e == cudaSuccess && occ < 1) e = cudaErrorInvalidConfiguration;
             bt->grid_c = bt->nsm * std::max(occ, 1);
+            if (e == cudaSuccess)
+                e = zstage::prepare(bt->all_quads ? batch_pass_a<true> : batch_pass_a<false>, 0, INT_MAX - 31, bt->nsm,
+                                    &bt->grid_a);
         }
         if (e != cudaSuccess) {
             delete bt;

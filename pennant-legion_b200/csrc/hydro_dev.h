@@ -72,11 +72,7 @@ struct DevArrays {
     float* cmass_f;
     float2* cforce_f;
     float2* sftot_f;
-    // batched meshes: per-tile partial reductions (npartA entries for pass
-    // A, npartC for C)
-    int32_t npartA, npartC;
-    double* part_dtnew;
-    int32_t* part_badA;
+    // batched meshes: pass C's partial reductions, one per zone tile
     double* part_dvov;
     int32_t* part_badC;
     // one mesh: the cycle's reductions, combined by every CTA of passes A

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kPointThreads) pass_b(DevArrays a, HydroConst 
     if (skip_cycle(ctl)) return;
     const int64_t p = (int64_t)blockIdx.x * kPointThreads + threadIdx.x;
     if (kRectPoints) {
-        if (p < a.nump) pass_b_point_rect<false>(a, c, ctl->cycle & 1, ctl->dt, p);
+        if (p < a.nump) pass_b_point_rect<false>(a, c, ctl->cycle & 1, ctl->dt, p, a.rect_nzx, a.numz / a.rect_nzx);
     } else {
         pass_b_point_csr<false>(a, c, ctl->cycle & 1, ctl->dt, p, p < a.nump);
     }

@@ -822,23 +822,25 @@ __device__ __forceinline__ void corner_values(const DevArrays& a, int64_t s, dou
     }
 }
 
-// A point of a rect mesh (a.rect_nzx > 0): its corners from its index, in
-// ascending side order from zero (Hydro.cc:1100-1116, :1175-1192).
+// A point of a rect-numbered mesh of nzx x nzy zones whose first point and
+// side are po and so: its corners from its index, in ascending side order
+// from zero (Hydro.cc:1100-1116, :1175-1192).
 template <bool kMixed>
 __device__ __forceinline__ void pass_b_point_rect(const DevArrays& a, const HydroConst& c, int cur, double dt,
-                                                  int64_t p) {
+                                                  int64_t p, int32_t nzx, int32_t nzy, int64_t po = 0,
+                                                  int64_t so = 0) {
     const double2 x0 = a.px[cur][p];
     const double2 u0 = a.pu[cur][p];
     double m = 0.;
     double2 f = mk(0., 0.);
     int64_t sc[4];
-    const int n = rect_point_corners(a.rect_nzx, a.numz / a.rect_nzx, p, sc);
+    const int n = rect_point_corners(nzx, nzy, p - po, sc);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         if (q < n) {
             double cm;
             double2 cf;
-            corner_values<kMixed>(a, sc[q], cm, cf);
+            corner_values<kMixed>(a, so + sc[q], cm, cf);
             m = __dadd_rn(m, cm);
             f = mk(__dadd_rn(f.x, cf.x), __dadd_rn(f.y, cf.y));
         }

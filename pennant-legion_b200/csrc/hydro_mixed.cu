@@ -28,6 +28,7 @@
 #include "closure_dev.cuh"
 #include "hydro_fp64_body.cuh"
 #include "batch_dev.h"
+#include "batch_tiles.cuh"
 #include "hydro_dev.h"
 #include "zone_stage.cuh"
 
@@ -79,23 +80,6 @@ __device__ __forceinline__ T zsum4(T v, int g, int n) {
 
 __device__ __forceinline__ bool skip_cycle(const Ctl* ctl) {
     return ctl->done || ctl->cycle >= ctl->stop_at;
-}
-
-template <bool kMin, int kThreads>
-__device__ __forceinline__ void block_fold(double v, double* out) {
-    __shared__ double red[kThreads / 32];
-    for (int o = 16; o > 0; o >>= 1) {
-        const double w = __shfl_xor_sync(kFull, v, o);
-        v = kMin ? dmin(v, w) : ((w > v) ? w : v);
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double r = red[0];
-        for (int i = 1; i < kThreads / 32; ++i) r = kMin ? dmin(r, red[i]) : ((red[i] > r) ? red[i] : r);
-        *out = r;
-    }
 }
 
 // ---------------------------------------------------------------------
@@ -173,15 +157,13 @@ __device__ __forceinline__ void qcs_sfq_fp64_zone(const DevArrays& a, const Hydr
     }
 }
 
-constexpr int kZoneThreadsZT = 128;   // pass A: one zone per thread
-
 // Per-side values parked in the thread's shared-memory slots between their
 // computation and their last use ([side][thread]: conflict-free).
 struct SideSpill {
     double2* sfp_;
     float2* sft_;
     int t;
-    int stride = kZoneThreadsZT;   // threads of the CTA
+    int stride;   // threads of the CTA
     __device__ __forceinline__ double2& sfp(int k) const { return sfp_[k * stride + t]; }
     __device__ __forceinline__ float2& sft(int k) const { return sft_[k * stride + t]; }
 };
@@ -471,56 +453,6 @@ __device__ __forceinline__ void pass_a_mixed_zone(const DevArrays& a, const Hydr
     }
 #pragma unroll
     for (int k = 0; k < N; ++k) a.cforce_f[s0 + k] = f2(sub(ftot[k], ftot[(k == 0) ? N - 1 : k - 1]));
-}
-
-#ifndef PNT_MIXED_ZT_MIN_BLOCKS
-#define PNT_MIXED_ZT_MIN_BLOCKS 4
-#endif
-
-template <bool kQuads, bool kLearned>
-__global__ void __launch_bounds__(kZoneThreadsZT, PNT_MIXED_ZT_MIN_BLOCKS) pass_a_mixed_zt(DevArrays a, HydroConst c) {
-    pdl_wait();
-    const Ctl* ctl = a.ctl;
-    if (skip_cycle(ctl)) return;
-    const int64_t z = (int64_t)blockIdx.x * kZoneThreadsZT + threadIdx.x;
-    double zdthyd = 1.e99;
-    int bad = 0;
-    int cnt[3] = {0, 0, 0};
-    __shared__ double2 s_sfp[4 * kZoneThreadsZT];
-    __shared__ float2 s_sft[4 * kZoneThreadsZT];
-    const SideSpill sp{s_sfp, s_sft, (int)threadIdx.x};
-    if (z < a.numz) {
-        const int cur = ctl->cycle & 1;
-        const double dt = ctl->dt;
-        const RecSink sink{a.closure_nrec, reinterpret_cast<float4*>(a.closure_rec), 0x7fffffff};
-        if (kQuads) {
-            const fp64::GlobalZoneIn in{a, cur, z, 4 * z};
-            pass_a_mixed_zone<4, kLearned>(a, c, in, cur, dt, z, 4 * z, zdthyd, bad, cnt, sp, sink);
-        } else {
-            const int n = a.znump[z];
-            const int64_t s0 = a.zfirst[z];
-            const fp64::GlobalZoneIn in{a, cur, z, s0};
-            if (n == 4) pass_a_mixed_zone<4, kLearned>(a, c, in, cur, dt, z, s0, zdthyd, bad, cnt, sp, sink);
-            else pass_a_mixed_zone<3, kLearned>(a, c, in, cur, dt, z, s0, zdthyd, bad, cnt, sp, sink);
-        }
-    }
-    __shared__ unsigned wcount[kLearned ? kZoneThreadsZT / 32 : 1][3];
-    if constexpr (kLearned) {
-        for (int q = 0; q < 3; ++q) {
-            const unsigned t = __reduce_add_sync(kFull, (unsigned)cnt[q]);
-            if ((threadIdx.x & 31) == 0) wcount[threadIdx.x >> 5][q] = t;
-        }
-    }
-    const int nbad = tiles::block_isum<kZoneThreadsZT>(bad);   // its barrier also orders wcount
-    if constexpr (kLearned) {
-        constexpr int kCounted[3] = {kClassZero, kClassDead, kClassAcute};
-        if (threadIdx.x < 3) {
-            unsigned t = 0;
-            for (int w = 0; w < kZoneThreadsZT / 32; ++w) t += wcount[w][threadIdx.x];
-            if (t) atomicAdd(a.closure_counts + kCounted[threadIdx.x] * 64 + (blockIdx.x & 63), (unsigned long long)t);
-        }
-    }
-    fp64::block_to_cycle<true, kZoneThreadsZT>(a.cyc_red, zdthyd, nbad);
 }
 
 // ---------------------------------------------------------------------
@@ -885,7 +817,7 @@ __global__ void __launch_bounds__(kPointThreads) pass_b_mixed(DevArrays a, Hydro
     if (skip_cycle(ctl)) return;
     const int64_t p = (int64_t)blockIdx.x * kPointThreads + threadIdx.x;
     if (kRect) {
-        if (p < a.nump) fp64::pass_b_point_rect<true>(a, c, ctl->cycle & 1, ctl->dt, p);
+        if (p < a.nump) fp64::pass_b_point_rect<true>(a, c, ctl->cycle & 1, ctl->dt, p, a.rect_nzx, a.numz / a.rect_nzx);
     } else {
         fp64::pass_b_point_csr<true>(a, c, ctl->cycle & 1, ctl->dt, p, p < a.nump);
     }
@@ -896,8 +828,16 @@ __global__ void __launch_bounds__(kPointThreads) pass_b_mixed(DevArrays a, Hydro
 // bodies above over the batch's work lists, as batch_pass_a and
 // batch_point_pass run the FP64 ones.
 // ---------------------------------------------------------------------
+// Pass A: one CTA a zone tile, plain loads, 16 warps an SM.  The warp walk of
+// the FP64 batch (btiles::for_tiles) was 5% faster while a batch's blasts are
+// small and 7% slower once many corners compress (12 instances of 48^2 to
+// 384^2 after 3000 cycles: 0.100 against 0.094 ms a cycle): the state of a
+// batch comes from L2, and tiles of acute zones hold up the warps they are
+// dealt to.
+constexpr int kBatchZT = 128;   // zones a step
 template <bool kAllQuads>
-__global__ void __launch_bounds__(kBatchZT, PNT_MIXED_ZT_MIN_BLOCKS) batch_pass_a_mixed(BatchDev b) {
+__global__ void __launch_bounds__(kBatchZT, 4) batch_pass_a_mixed(BatchDev b) {
+    pdl_wait();
     const int t = blockIdx.x;
     if (t >= b.nztiles) return;   // no tiles left: the grid is one idle CTA
     const Tile tile = b.ztiles[t];
@@ -908,9 +848,9 @@ __global__ void __launch_bounds__(kBatchZT, PNT_MIXED_ZT_MIN_BLOCKS) batch_pass_
     const double dt = ctl.dt;
     __shared__ double2 s_sfp[4 * kBatchZT];
     __shared__ float2 s_sft[4 * kBatchZT];
-    const SideSpill sp{s_sfp, s_sft, (int)threadIdx.x};
-    double fold = 1.e99;
-    int nbad = 0;
+    const SideSpill sp{s_sfp, s_sft, (int)threadIdx.x, kBatchZT};
+    btiles::InstFold fold;
+    fold.inst = tile.inst;
     for (int zb = tile.beg; zb < tile.end; zb += kBatchZT) {
         const int64_t z = (int64_t)zb + threadIdx.x;
         if (z >= tile.end) continue;
@@ -918,22 +858,22 @@ __global__ void __launch_bounds__(kBatchZT, PNT_MIXED_ZT_MIN_BLOCKS) batch_pass_
         int cnt[3] = {0, 0, 0};
         if (kAllQuads || tile.quads) {
             const fp64::GlobalZoneIn in{b.a, cur, z, 4 * z};
-            pass_a_mixed_zone<4, false>(b.a, c, in, cur, dt, z, 4 * z, v, nbad, cnt, sp);
+            pass_a_mixed_zone<4, false>(b.a, c, in, cur, dt, z, 4 * z, v, fold.bad, cnt, sp);
         } else {
             const int n = b.a.znump[z];
             const int64_t s0 = b.a.zfirst[z];
             const fp64::GlobalZoneIn in{b.a, cur, z, s0};
-            if (n == 4) pass_a_mixed_zone<4, false>(b.a, c, in, cur, dt, z, s0, v, nbad, cnt, sp);
-            else pass_a_mixed_zone<3, false>(b.a, c, in, cur, dt, z, s0, v, nbad, cnt, sp);
+            if (n == 4) pass_a_mixed_zone<4, false>(b.a, c, in, cur, dt, z, s0, v, fold.bad, cnt, sp);
+            else pass_a_mixed_zone<3, false>(b.a, c, in, cur, dt, z, s0, v, fold.bad, cnt, sp);
         }
-        fold = dmin(fold, v);
+        fold.v = dmin(fold.v, v);
     }
-    nbad = tiles::block_isum<kBatchZT>(nbad);
-    block_fold<true, kBatchZT>(fold, b.a.part_dtnew + t);
-    if (threadIdx.x == 0) b.a.part_badA[t] = nbad;
+    __syncwarp();
+    fold.flush(b);
 }
 
 __global__ void __launch_bounds__(kBatchThreads) batch_point_pass_mixed(BatchDev b) {
+    pdl_wait();
     for (int t = blockIdx.x; t < b.nptiles; t += gridDim.x) {
         const Tile tile = b.ptiles[t];
         const Ctl& ctl = b.ctls[tile.inst];
@@ -942,7 +882,13 @@ __global__ void __launch_bounds__(kBatchThreads) batch_point_pass_mixed(BatchDev
         const int cur = ctl.cycle & 1;
         for (int64_t pb = tile.beg; pb < tile.end; pb += kBatchThreads) {
             const int64_t p = pb + threadIdx.x;
-            fp64::pass_b_point_csr<true>(b.a, c, cur, ctl.dt, p, p < tile.end);
+            if (tile.nzx > 0) {
+                if (p < tile.end)
+                    fp64::pass_b_point_rect<true>(b.a, c, cur, ctl.dt, p, tile.nzx, tile.nzy, tile.po,
+                                                  4 * (int64_t)tile.zo);
+            } else {
+                fp64::pass_b_point_csr<true>(b.a, c, cur, ctl.dt, p, p < tile.end);
+            }
         }
     }
 }
@@ -1022,14 +968,13 @@ cudaError_t prepare_pass_a_mixed(bool learned, int32_t rect_nzx, bool quads, int
     return zstage::prepare(pass_a_kernel(learned, rect_nzx, quads), rect_nzx, numz, nsm, grid);
 }
 
-void launch_batch_pass_a_mixed(const BatchDev& b, bool all_quads, cudaStream_t stream) {
-    const int grid = b.nztiles > 1 ? b.nztiles : 1;
-    if (all_quads) batch_pass_a_mixed<true><<<grid, kBatchZT, 0, stream>>>(b);
-    else batch_pass_a_mixed<false><<<grid, kBatchZT, 0, stream>>>(b);
+cudaError_t launch_batch_pass_a_mixed(const BatchDev& b, bool all_quads, cudaStream_t stream) {
+    return launch_pdl(all_quads ? batch_pass_a_mixed<true> : batch_pass_a_mixed<false>, b.nztiles > 1 ? b.nztiles : 1,
+                      kBatchZT, 0, stream, b);
 }
 
-void launch_batch_point_pass_mixed(const BatchDev& b, int grid, cudaStream_t stream) {
-    batch_point_pass_mixed<<<grid, kBatchThreads, 0, stream>>>(b);
+cudaError_t launch_batch_point_pass_mixed(const BatchDev& b, int grid, cudaStream_t stream) {
+    return launch_pdl(batch_point_pass_mixed, grid, kBatchThreads, 0, stream, b);
 }
 
 cudaError_t prepare_learned_kernels() {
