@@ -298,6 +298,7 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
     int32_t *zfirst = nullptr, *znump = nullptr, *mapsp1 = nullptr, *poff = nullptr, *pcorner = nullptr;
     double* smf = nullptr;
     uint16_t* mask = nullptr;
+    uint8_t* zone_bc = nullptr;
     // the persistent pass C's grid
     {
         int nsm = 148;
@@ -317,7 +318,7 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
     pnt_status st = PNT_OK;
     if ((st = h->alloc(&zfirst, nz)) || (st = h->alloc(&znump, nz)) || (st = h->alloc(&mapsp1, ns)) ||
         (st = h->alloc(&smf, ns)) || (st = h->alloc(&poff, np + 1)) || (st = h->alloc(&pcorner, m.pcorner.size())) ||
-        (st = h->alloc(&mask, np + 2)) || (st = h->alloc(&a.px[0], np)) || (st = h->alloc(&a.px[1], np)) ||
+        (st = h->alloc(&mask, np + 2)) || (st = h->alloc(&zone_bc, nz)) || (st = h->alloc(&a.px[0], np)) || (st = h->alloc(&a.px[1], np)) ||
         (st = h->alloc(&a.pu[0], np)) || (st = h->alloc(&a.pu[1], np)) || (st = h->alloc(&a.zm, nz + 2)) ||
         (st = h->alloc(&a.zr, nz + 2)) || (st = h->alloc(&a.ze, nz + 2)) || (st = h->alloc(&a.zetot, nz + 2)) ||
         (st = h->alloc(&a.zwrate, nz + 2)) || (st = h->alloc(&a.zvol, nz + 2)) || (st = h->alloc(&a.zp, nz + 2)) ||
@@ -334,6 +335,7 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
     a.poff = poff;
     a.pcorner = pcorner;
     a.bcmask = mask;
+    a.zone_bc = zone_bc;
     if (m.is_piece) {
         // a piece: halo corner slots follow the local sides in cmass/cforce
         h->piece = true;
@@ -392,6 +394,8 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
         (e = cudaMemsetAsync(a.px[1], 0, np * 16, s)) ||
         (e = cudaMemsetAsync(a.pu[1], 0, np * 16, s)))
         return fail(PNT_ERR_CUDA, "memset: %s", cudaGetErrorString(e));
+    if (a.rect_nzx > 0 && (e = launch_find_zone_bc(a, zone_bc, s)))
+        return fail(PNT_ERR_CUDA, "boundary zones: %s", cudaGetErrorString(e));
     CUDA_TRY(cudaStreamSynchronize(s));
     *h->ctl_host = ctl;
     return PNT_OK;

@@ -55,6 +55,7 @@ struct DevArrays {
     const int32_t* poff;         // [nump+1]
     const int32_t* pcorner;      // [nums]
     const uint16_t* bcmask;      // [nump] bit b: point on BC plane b
+    const uint8_t* zone_bc;      // [numz] the zone has a point on a BC plane (pass C on rect meshes)
     double2* px[2];              // point position, double buffered by cycle parity
     double2* pu[2];              // point velocity
     double* zm;
@@ -179,6 +180,8 @@ cudaError_t prepare_learned_kernels();
 // write a.gridC partials.
 cudaError_t prepare_pass_c(bool mixed, bool quads, int32_t rect_nzx, int32_t numz, int nsm, int32_t* grid);
 void launch_pass_c(const DevArrays& a, const HydroConst& c, bool mixed, cudaStream_t stream);
+// a.zone_bc from the mesh and the points' masks (pass_c.cu).
+cudaError_t launch_find_zone_bc(const DevArrays& a, uint8_t* zone_bc, cudaStream_t stream);
 // Pass A of the FP64 cycle (hydro_fp64.cu) and of the mixed or learned cycle
 // (hydro_mixed.cu): raises the kernel's shared-memory limit on the current
 // device and returns its persistent grid (and the tiles a.redo holds a word

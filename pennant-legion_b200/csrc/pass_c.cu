@@ -18,12 +18,16 @@ namespace {
 // Pass C over row tiles of a rect mesh (row_tiles.cuh): per tile of up to
 // kRowT zones, the bottom and top point rows of px0, pu0, px, pu and four
 // zone fields arrive by bulk copies; each thread reads its zone's sfp + sfq
-// (64 contiguous bytes) and the BC plane masks (two bytes a point, cached)
-// from global memory.  64 zones and two stages a CTA, shared memory for 10
-// CTAs an SM: 1920^2 Sedov 0.149 ms, against 0.163 ms with sfp + sfq in the
-// stages (7 CTAs an SM), 0.152 ms with the zone fields also from global
-// memory, 0.174-0.185 ms with three stages and 0.173 ms for the staged
-// gathers.
+// (64 contiguous bytes) from global memory, and the BC plane masks where its
+// zone has a point on a plane (a flag a zone, read a tile ahead: the masks of
+// every zone were a second memory latency a tile).  64 zones and two stages a
+// CTA, shared memory for 10 CTAs an SM.  Bound by latency and HBM: 1920^2
+// Sedov 0.135 ms (its 190 bytes a zone take 0.107 ms); 0.146 ms with the masks
+// of every zone and the division operator, 0.150 ms without the prefetch of
+// sfp + sfq into L2 too; that one against 0.163 ms with sfp + sfq in the stages
+// (7 CTAs an SM), 0.152 ms with the zone fields also from global memory,
+// 0.174-0.185 ms with three stages or sfp + sfq held a tile ahead in registers
+// (8 CTAs) and 0.173 ms for the staged gathers.
 // ---------------------------------------------------------------------
 #ifndef PNT_ROWS_C_T
 #define PNT_ROWS_C_T 64
@@ -40,7 +44,13 @@ constexpr int kRowStageBytes = kRowOffZs + 4 * kRowZB;
 constexpr int kRowSmemBytes = kRowStages * kRowStageBytes;
 static_assert(kRowT % 2 == 0 && kRowStageBytes % 16 == 0, "16-byte aligned stages");
 
+// From here on the sfp + sfq of a mesh do not stay in L2 until pass C and are
+// prefetched a tile ahead (1920^2: 0.150 -> 0.146 ms; at 480^2, where they do
+// stay, the prefetch cost 2%).
+constexpr int32_t kPrefetchZones = 500000;
+
 struct RowIn {
+    static constexpr bool kStraight = true;
     const unsigned char* st;
     const uint16_t* bcmask;
     int64_t pb, npx;
@@ -56,6 +66,8 @@ struct RowIn {
     __device__ __forceinline__ double2 u(int k) const { return *f(3, k); }
     const double2* sfg;   // the zone's sfp + sfq (global memory)
     __device__ __forceinline__ double2 sf(int k) const { return sfg[k]; }
+    bool any_bc;          // a point of the zone is on a BC plane
+    __device__ __forceinline__ bool bc() const { return any_bc; }
     __device__ __forceinline__ unsigned mask(int k) const { return __ldg(bcmask + pb + row(k) * npx + col(k)); }
     __device__ __forceinline__ double zs(int fld) const {
         return reinterpret_cast<const double*>(st + kRowOffZs + fld * kRowZB)[shift + t];
@@ -104,10 +116,23 @@ __global__ void __launch_bounds__(kRowT) pass_c_rows(DevArrays a, HydroConst c) 
         for (int f = 0; f < 4; ++f)
             rows::bulk_g2s(st + kRowOffZs + f * kRowZB, zf[f] + zr.zs, (uint32_t)(zr.count * 8), bar);
     };
+    // whether the thread's zone of tile g has a point on a BC plane, a tile
+    // ahead; and the next tile's sfp + sfq into L2
+    const bool far = a.numz > kPrefetchZones;
+    auto look_ahead = [&](int64_t g) -> uint8_t {
+        if (g >= ntiles) return 0;
+        const rows::Tile tn = rows::tile_of<kRowT>(g, nzx);
+        if (t >= tn.nt) return 0;
+        if (far) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.sftot + 4 * (tn.z0 + t)));
+        return __ldg(a.zone_bc + tn.z0 + t);
+    };
+    uint8_t bc_next = look_ahead(blockIdx.x);
     auto compute = [&](const unsigned char* st, int64_t g) {
         const rows::Tile tl = rows::tile_of<kRowT>(g, nzx);
+        const bool bc = bc_next != 0;
+        bc_next = look_ahead(g + gridDim.x);
         if (t >= tl.nt) return;
-        const RowIn in{st, a.bcmask, tl.pb, npx, t, (int)(tl.z0 & 1), a.sftot + 4 * (tl.z0 + t)};
+        const RowIn in{st, a.bcmask, tl.pb, npx, t, (int)(tl.z0 & 1), a.sftot + 4 * (tl.z0 + t), bc};
         const double d = stagedc::zone_core<true, kMixed>(a, c, 4, in, tl.z0 + t, dt, dtinv, nbad);
         dvm = (d > dvm) ? d : dvm;
     };
@@ -130,6 +155,15 @@ __global__ void __launch_bounds__(stagedc::kTile) pass_c_staged(DevArrays a, Hyd
     const int nb = tiles::block_isum<stagedc::kTile>(nbad);
     fp64::block_to_cycle<false, stagedc::kTile>(a.cyc_red, dvm, nb);
     fp64::end_cycle_if_last(a, c);
+}
+
+// Which zones have a point on a BC plane.
+__global__ void find_zone_bc(DevArrays a, uint8_t* zone_bc) {
+    const int64_t z = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (z >= a.numz) return;
+    unsigned m = 0;
+    for (int k = 0; k < a.znump[z]; ++k) m |= a.bcmask[a.mapsp1[a.zfirst[z] + k]];
+    zone_bc[z] = m ? 1 : 0;
 }
 
 using Kernel = void (*)(DevArrays, HydroConst);
@@ -157,6 +191,11 @@ cudaError_t prepare_pass_c(bool mixed, bool quads, int32_t rect_nzx, int32_t num
         return cudaSuccess;
     }
     return tiles::prepare(pick_kernel(mixed, quads), stagedc::kTile, stagedc::kSmemBytes, numz, nsm, grid);
+}
+
+cudaError_t launch_find_zone_bc(const DevArrays& a, uint8_t* zone_bc, cudaStream_t stream) {
+    find_zone_bc<<<(unsigned)((a.numz + 255) / 256), 256, 0, stream>>>(a, zone_bc);
+    return cudaGetLastError();
 }
 
 void launch_pass_c(const DevArrays& a, const HydroConst& c, bool mixed, cudaStream_t stream) {
