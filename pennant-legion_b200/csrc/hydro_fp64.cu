@@ -100,17 +100,17 @@ __global__ void __launch_bounds__(32, 8) pass_a(DevArrays a, HydroConst c) {
     warp_to_cycle<true>(a.cyc_red, zdthyd, bad);
 }
 
-// Pass A of a small mesh: four lanes a zone, eight zones a warp, one warp a
-// CTA.
+// Pass A of a small mesh: four lanes a zone, 32 zones a CTA.
+constexpr int kSmallThreads = 128;
 template <MeshKind kKind>
-__global__ void __launch_bounds__(32) pass_a_small(DevArrays a, HydroConst c) {
+__global__ void __launch_bounds__(kSmallThreads) pass_a_small(DevArrays a, HydroConst c) {
     pdl_wait();
     const Ctl* ctl = a.ctl;
     if (skip_cycle(ctl)) return;
     const int cur = ctl->cycle & 1;
     const double dt = ctl->dt;
-    const int lane = threadIdx.x;
-    const int zl = (int)blockIdx.x * 8 + (lane >> 2);
+    const int lane = threadIdx.x & 31;
+    const int zl = (int)(blockIdx.x * kSmallThreads + threadIdx.x) >> 2;
     const bool live = zl < a.numz;
     const int z = live ? zl : a.numz - 1;
     const zstage::Idx ix =
@@ -129,7 +129,8 @@ __global__ void __launch_bounds__(32) pass_a_small(DevArrays a, HydroConst c) {
         }
     }
     __syncwarp();
-    warp_to_cycle<true>(a.cyc_red, zdthyd, bad);
+    const int nbad = tiles::block_isum<kSmallThreads>(bad);
+    block_to_cycle<true, kSmallThreads>(a.cyc_red, zdthyd, nbad);
 }
 
 template <bool kRectPoints>
@@ -202,7 +203,7 @@ cudaError_t launch_cycle_fp64(const DevArrays& a, const HydroConst& c, cudaStrea
         if (ev) cudaEventRecord(ev[0], stream);
         if (a.numz <= kSmallZones)
             e = launch_pdl(a.rect_nzx > 0 ? pass_a_small<kRect> : (a.quads ? pass_a_small<kQuads> : pass_a_small<kGeneral>),
-                           (a.numz + 7) / 8, 32, 0, stream, a, c);
+                           (a.numz + kSmallThreads / 4 - 1) / (kSmallThreads / 4), kSmallThreads, 0, stream, a, c);
         else
             e = launch_pdl(pass_a_kernel(a.rect_nzx, a.quads != 0), a.gridA, 32, zstage::kSmem, stream, a, c);
         if (ev) cudaEventRecord(ev[1], stream);

@@ -101,6 +101,41 @@ __device__ __forceinline__ double2 proj(double2 v, double ux, double uy) {
     return mk2(v.x - ux * d, v.y - uy * d);
 }
 
+// The end of a zone's corrector from its new volume, energy and work: writes
+// zvol, zr, zetot, ze, zwrate and returns |dV/V0|.
+template <bool kStraight>
+__device__ __forceinline__ double zone_results(const DevArrays& a, int64_t z, double zm, double zvol0, double zp,
+                                               double dtinv, double zvol, double zetot, double zw) {
+    // calcWorkRate (Hydro.cc:1483-1510), calcEnergy (:1545-1564),
+    // calcRho (:1034-1054), calcDvol (:1622-1644)
+    const double dvol = zvol - zvol0;
+    const double zwrate = (zw + zp * dvol) * dtinv;
+    const double zme = zm + 1.e-99;
+    double zr, ze, dv;
+    // the three quotients in straight-line code, where the kernel gains from
+    // it, or with the operators (also where an operand is out of the range of
+    // ieee_div.cuh)
+    bool ops = true;
+    if constexpr (kStraight) {
+        ieee::Guard g;
+        zr = ieee::quot(zm, zvol, ieee::rcp(zvol, g), g);
+        ze = ieee::quot0(zetot, zme, ieee::rcp(zme, g), g);
+        dv = ieee::quot0(dvol, zvol0, ieee::rcp(zvol0, g), g);
+        ops = !g.ok();
+    }
+    if (ops) {
+        zr = zm / zvol;
+        ze = zetot / zme;
+        dv = dvol / zvol0;
+    }
+    a.zvol[z] = zvol;
+    a.zr[z] = zr;
+    a.zetot[z] = zetot;
+    a.ze[z] = ze;
+    a.zwrate[z] = zwrate;
+    return fabs(dv);
+}
+
 // One zone's corrector from its inputs, read through `in` where they are
 // used: for side k < n, in.x(k) / in.u(k) the new position and velocity of
 // the side's first point, in.u0(k) its start-of-cycle velocity (before the
@@ -181,34 +216,7 @@ __device__ __forceinline__ double zone_core(const DevArrays& a, const HydroConst
         }
     }
     if (kMixed) zetot = zetot0 + zw;
-    // calcWorkRate (Hydro.cc:1483-1510), calcEnergy (:1545-1564),
-    // calcRho (:1034-1054), calcDvol (:1622-1644)
-    const double dvol = zvol - zvol0;
-    const double zwrate = (zw + zp * dvol) * dtinv;
-    const double zme = zm + 1.e-99;
-    double zr, ze, dv;
-    // the three quotients in straight-line code, where the kernel gains from
-    // it, or with the operators (also where an operand is out of the range of
-    // ieee_div.cuh)
-    bool ops = true;
-    if constexpr (In::kStraight) {
-        ieee::Guard g;
-        zr = ieee::quot(zm, zvol, ieee::rcp(zvol, g), g);
-        ze = ieee::quot0(zetot, zme, ieee::rcp(zme, g), g);
-        dv = ieee::quot0(dvol, zvol0, ieee::rcp(zvol0, g), g);
-        ops = !g.ok();
-    }
-    if (ops) {
-        zr = zm / zvol;
-        ze = zetot / zme;
-        dv = dvol / zvol0;
-    }
-    a.zvol[z] = zvol;
-    a.zr[z] = zr;
-    a.zetot[z] = zetot;
-    a.ze[z] = ze;
-    a.zwrate[z] = zwrate;
-    return fabs(dv);
+    return zone_results<In::kStraight>(a, z, zm, zvol0, zp, dtinv, zvol, zetot, zw);
 }
 
 // The staged layout above, slot t of stage st; sfg: the zone's sfp + sfq
