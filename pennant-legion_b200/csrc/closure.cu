@@ -337,13 +337,28 @@ __global__ void pack_images(const float* P, Norm nm, float thr0, float thr1, flo
     }
 }
 
-// Sum of the per-CTA partials (fixed order); Adam step when `apply`.
-__global__ void closure_reduce_adam(float* params, float* m, float* v, const float* partial, int nparts, float lr,
-                                    float bc1, float bc2, float inv_count, int apply, float* grad_out, float* loss_out) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p > kClParams) return;
+// Sum of the per-CTA partials (fixed order); Adam step when `apply`.  32
+// parameters a CTA, each by 8 threads that sum every 8th partial and are
+// then added in order: one thread a parameter waited for a gather from L2
+// every few of the partials (256 in a 32768-row step).
+constexpr int kReduceThreads = 256;
+constexpr int kReduceSplit = 8;
+__global__ void __launch_bounds__(kReduceThreads)
+    closure_reduce_adam(float* params, float* m, float* v, const float* partial, int nparts, float lr, float bc1,
+                        float bc2, float inv_count, int apply, float* grad_out, float* loss_out) {
+    __shared__ float part[kReduceSplit][32];
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+    const int p = blockIdx.x * 32 + lane;
     float s = 0.f;
-    for (int b = 0; b < nparts; ++b) s += partial[(int64_t)b * (kClParams + 1) + p];
+    if (p <= kClParams) {
+#pragma unroll 8
+        for (int b = q; b < nparts; b += kReduceSplit) s += partial[(int64_t)b * (kClParams + 1) + p];
+    }
+    part[q][lane] = s;
+    __syncthreads();
+    if (q > 0 || p > kClParams) return;
+#pragma unroll
+    for (int i = 1; i < kReduceSplit; ++i) s += part[i][lane];
     if (p == kClParams) {
         *loss_out = s * inv_count;
         return;
@@ -546,7 +561,7 @@ struct pnt_closure {
             bc1 = 1.f - powf(0.9f, (float)adam_t);
             bc2 = 1.f - powf(0.999f, (float)adam_t);
         }
-        closure_reduce_adam<<<(kClParams + 1 + 255) / 256, 256, 0, stream>>>(
+        closure_reduce_adam<<<(kClParams + 1 + 31) / 32, kReduceThreads, 0, stream>>>(
             d_params, d_m, d_v, d_partial, nparts, lr, bc1, bc2, A.inv_count, apply ? 1 : 0,
             grad_host ? d_grad : nullptr, d_loss);
         CUDA_TRY(cudaGetLastError());

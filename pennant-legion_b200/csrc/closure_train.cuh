@@ -35,7 +35,10 @@
 namespace pnt {
 namespace train {
 
-constexpr int kThreads = 128;
+// Two threads a row: threads t and t + 128 take the two halves of row t's
+// columns in every epilogue (their warps, w and w + 4, share the TMEM lanes).
+// The epilogues, 256 GELUs a row, are what the kernel spends its time on.
+constexpr int kThreads = 256;
 constexpr int kRows = 128;
 
 // Training image in global memory (bf16 operands in the canonical layout;
@@ -142,20 +145,20 @@ struct Tc {
         tc_fence_after();
     }
     __device__ __forceinline__ uint32_t lane_addr(uint32_t col) const {
-        return tbase + ((uint32_t)(32 * (threadIdx.x >> 5)) << 16) + col;
+        return tbase + ((uint32_t)(32 * ((threadIdx.x >> 5) & 3)) << 16) + col;
     }
 };
 
 __global__ void __launch_bounds__(kThreads, 1) grad_kernel(Args A) {
     extern __shared__ __align__(1024) uint8_t sm[];
-    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    const int tid = threadIdx.x, half = tid >> 7, t = tid & 127, w = t >> 5, lane = tid & 31;
     // ---- setup: image, this thread's row of X (and X^T), zero paddings
-    for (int i = t; i < kImgBytes / 16; i += kThreads)
+    for (int i = tid; i < kImgBytes / 16; i += kThreads)
         reinterpret_cast<uint4*>(sm + kSImg)[i] = __ldg(reinterpret_cast<const uint4*>(A.img) + i);
     const int64_t idx = (int64_t)blockIdx.x * kRows + t;
     const bool live = idx < A.rows;
     const int64_t row = live ? (A.first + idx) % A.n : 0;
-    {
+    if (half == 0) {
         uint4 v0 = make_uint4(0u, 0u, 0u, 0u), v1 = v0;
         if (live) {
             v0 = __ldg(reinterpret_cast<const uint4*>(A.x + row * 16));
@@ -171,12 +174,12 @@ __global__ void __launch_bounds__(kThreads, 1) grad_kernel(Args A) {
             *reinterpret_cast<__nv_bfloat16*>(sm + kSXT + canon(8 + i, t, 16)) = xv1[i];
         }
     }
-    for (int i = t; i < 64 * 128 * 2 / 16; i += kThreads)   // T2 rows 64-127 (k-chunks interleave rows)
+    for (int i = tid; i < 64 * 128 * 2 / 16; i += kThreads)   // T2 rows 64-127 (k-chunks interleave rows)
         reinterpret_cast<uint4*>(sm + kST2)[(i / 64) * 128 + 64 + (i % 64)] = make_uint4(0u, 0u, 0u, 0u);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kSBar + 8);
     Tc tc{(uint32_t)__cvta_generic_to_shared(sm), (uint32_t)__cvta_generic_to_shared(sm + kSBar), 0u, 0u, true};
-    if (t == 0) mbar_init(tc.mbar, 1);
-    if (w == 0) {
+    if (tid == 0) mbar_init(tc.mbar, 1);
+    if (tid < 32) {
         tmem_alloc((uint32_t)__cvta_generic_to_shared(tslot), kTmemCols);
         tmem_relinquish();
     }
@@ -189,11 +192,11 @@ __global__ void __launch_bounds__(kThreads, 1) grad_kernel(Args A) {
     float loss = 0.f;
 
     // ---- layer 1
-    if (t == 0) tc.mma(kD1, kSX, 128, kImgW1, 64, 1, 0);
+    if (tid == 0) tc.mma(kD1, kSX, 128, kImgW1, 64, 1, 0);
     tc.commit_wait();
     if (tc.ok) {
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 2 * half; c < 2 * half + 2; ++c) {
             float v[16], h[16];
             tmem_ld16(tc.lane_addr(kD1 + 16 * c), v);
 #pragma unroll
@@ -208,11 +211,11 @@ __global__ void __launch_bounds__(kThreads, 1) grad_kernel(Args A) {
     }
     tc.publish();
     // ---- layer 2
-    if (t == 0 && tc.ok) tc.mma(kD2, kSH1, 128, kImgW2, 64, 4, 0);
+    if (tid == 0 && tc.ok) tc.mma(kD2, kSH1, 128, kImgW2, 64, 4, 0);
     tc.commit_wait();
     if (tc.ok) {
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 2 * half; c < 2 * half + 2; ++c) {
             float v[16], h[16];
             tmem_ld16(tc.lane_addr(kD2 + 16 * c), v);
 #pragma unroll
@@ -227,11 +230,11 @@ __global__ void __launch_bounds__(kThreads, 1) grad_kernel(Args A) {
     }
     tc.publish();
     // ---- layer 3, loss, dY
-    if (t == 0 && tc.ok) tc.mma(kD3, kSH2, 128, kImgW3, 16, 4, 0);
+    if (tid == 0 && tc.ok) tc.mma(kD3, kSH2, 128, kImgW3, 16, 4, 0);
     tc.commit_wait();
     float dy[16];
     for (int i = 0; i < 16; ++i) dy[i] = 0.f;
-    if (tc.ok) {
+    if (tc.ok && half == 0) {
         float v[4];
         tmem_ld4(tc.lane_addr(kD3), v);
         if (live) {
@@ -249,17 +252,17 @@ __global__ void __launch_bounds__(kThreads, 1) grad_kernel(Args A) {
         st_row8(sm + kSDY, t, 0, dy);
         st_row8(sm + kSDY, t, 1, dy + 8);
     }
-    {
+    if (half == 0) {
         warp_colsum16(dy);   // the bias gradient of layer 3 (FP32, unrounded)
         if (lane == 0)
             for (int o = 0; o < 4; ++o) bsum[128 + o] = dy[o];
     }
     tc.publish();
     // ---- dZ2 = (dY W3) gelu'(Z2)
-    if (t == 0 && tc.ok) tc.mma(kD4, kSDY, 128, kImgW3T, 64, 1, 0);
+    if (tid == 0 && tc.ok) tc.mma(kD4, kSDY, 128, kImgW3T, 64, 1, 0);
     tc.commit_wait();
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 2 * half; c < 2 * half + 2; ++c) {
         float dz[16];
         for (int i = 0; i < 16; ++i) dz[i] = 0.f;
         if (tc.ok) {
@@ -282,10 +285,10 @@ __global__ void __launch_bounds__(kThreads, 1) grad_kernel(Args A) {
     }
     tc.publish();
     // ---- dZ1 = (dZ2 W2) gelu'(Z1)
-    if (t == 0 && tc.ok) tc.mma(kD5, kSDZ2, 128, kImgW2T, 64, 4, 0);
+    if (tid == 0 && tc.ok) tc.mma(kD5, kSDZ2, 128, kImgW2T, 64, 4, 0);
     tc.commit_wait();
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 2 * half; c < 2 * half + 2; ++c) {
         float dz[16];
         for (int i = 0; i < 16; ++i) dz[i] = 0.f;
         if (tc.ok) {
@@ -306,10 +309,10 @@ __global__ void __launch_bounds__(kThreads, 1) grad_kernel(Args A) {
     }
     // the loss: the warp's rows, then the warps in order below
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-    if (lane == 0) reinterpret_cast<float*>(sm + kSLoss)[w] = loss;
+    if (lane == 0 && half == 0) reinterpret_cast<float*>(sm + kSLoss)[w] = loss;
     tc.publish();
     // ---- weight gradients: contractions over the CTA's 128 rows
-    if (t == 0 && tc.ok) {
+    if (tid == 0 && tc.ok) {
         tc.mma(kG1, kST1, 128, kSH1T, 64, 8, 0);
         tc.mma(kG2, kST1, 128, kSXT, 16, 8, 0);
         tc.mma(kG3, kST2, 128, kSDYT, 16, 8, 0);
@@ -317,29 +320,31 @@ __global__ void __launch_bounds__(kThreads, 1) grad_kernel(Args A) {
     tc.commit_wait();
     float* P = A.partial + (int64_t)blockIdx.x * (kClParams + 1);
     if (w < 2) {   // rows 0-63: dW2[j][.] and dW3[.][j], j = t
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 2 * half; c < 2 * half + 2; ++c) {
             float v[16];
             if (tc.ok) tmem_ld16(tc.lane_addr(kG1 + 16 * c), v);
             for (int i = 0; i < 16; ++i) P[kClW2 + t * 64 + 16 * c + i] = tc.ok ? v[i] : __int_as_float(0x7fc00000);
         }
-        float v[4];
-        if (tc.ok) tmem_ld4(tc.lane_addr(kG3), v);
-        for (int o = 0; o < kClOut; ++o) P[kClW3 + o * 64 + t] = tc.ok ? v[o] : __int_as_float(0x7fc00000);
-    } else {       // rows 64-127: dW1[j][.], j = t - 64
+        if (half == 0) {
+            float v[4];
+            if (tc.ok) tmem_ld4(tc.lane_addr(kG3), v);
+            for (int o = 0; o < kClOut; ++o) P[kClW3 + o * 64 + t] = tc.ok ? v[o] : __int_as_float(0x7fc00000);
+        }
+    } else if (half == 0) {       // rows 64-127: dW1[j][.], j = t - 64
         float v[16];
         if (tc.ok) tmem_ld16(tc.lane_addr(kG2), v);
         for (int i = 0; i < kClIn; ++i) P[kClW1 + (t - 64) * kClIn + i] = tc.ok ? v[i] : __int_as_float(0x7fc00000);
     }
     // ---- biases (warps summed in order) and the loss
     const float* bs = reinterpret_cast<const float*>(sm + kSBias);
-    for (int i = t; i < 132; i += kThreads) {
+    for (int i = tid; i < 132; i += kThreads) {
         if (i >= 128 + kClOut) continue;
         const float s = ((bs[i] + bs[132 + i]) + bs[264 + i]) + bs[396 + i];
         if (i < 64) P[kClB1 + i] = s;
         else if (i < 128) P[kClB2 + i - 64] = s;
         else P[kClB3 + i - 128] = s;
     }
-    if (t == 0) {
+    if (tid == 0) {
         const float* ls = reinterpret_cast<const float*>(sm + kSLoss);
         P[kClParams] = tc.ok ? ((ls[0] + ls[1]) + ls[2]) + ls[3] : __int_as_float(0x7fc00000);
         if (!tc.ok) atomicOr(A.err, 1);
@@ -351,7 +356,7 @@ __global__ void __launch_bounds__(kThreads, 1) grad_kernel(Args A) {
         mbar_wait(tc.mbar, (tc.phase - 1) & 1);
         __syncthreads();
     }
-    if (w == 0) {
+    if (tid < 32) {
         tc_fence_after();
         tmem_dealloc(tc.tbase, kTmemCols);
     }

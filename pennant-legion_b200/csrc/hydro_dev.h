@@ -55,7 +55,6 @@ struct DevArrays {
     const int32_t* poff;         // [nump+1]
     const int32_t* pcorner;      // [nums]
     const uint16_t* bcmask;      // [nump] bit b: point on BC plane b
-    const uint8_t* zone_bc;      // [numz] the zone has a point on a BC plane (pass C on rect meshes)
     double2* px[2];              // point position, double buffered by cycle parity
     double2* pu[2];              // point velocity
     double* zm;
@@ -100,6 +99,7 @@ struct DevArrays {
     // -dvovmax, inverted sides in A, in C] here instead of ending the cycle
     // (nullptr for a single piece)
     double* piece_red;
+    const uint8_t* zone_bc;   // [numz] the zone has a point on a BC plane (pass C on rect meshes)
 };
 
 constexpr int kZoneThreads = 256;   // pass A: 64 zones x 4 side lanes per block

@@ -68,8 +68,9 @@ struct RowIn {
     const double2* sfg;   // the zone's sfp + sfq (global memory)
     __device__ __forceinline__ double2 sf(int k) const { return sfg[k]; }
     bool any_bc;          // a point of the zone is on a BC plane
-    __device__ __forceinline__ bool bc() const { return any_bc; }
-    __device__ __forceinline__ unsigned mask(int k) const { return __ldg(bcmask + pb + row(k) * npx + col(k)); }
+    __device__ __forceinline__ unsigned mask(int k) const {
+        return any_bc ? __ldg(bcmask + pb + row(k) * npx + col(k)) : 0u;
+    }
     __device__ __forceinline__ double zs(int fld) const {
         return reinterpret_cast<const double*>(st + kRowOffZs + fld * kRowZB)[shift + t];
     }

@@ -110,37 +110,40 @@ __device__ __forceinline__ double zone_results(const DevArrays& a, int64_t z, do
     // calcRho (:1034-1054), calcDvol (:1622-1644)
     const double dvol = zvol - zvol0;
     const double zwrate = (zw + zp * dvol) * dtinv;
-    const double zme = zm + 1.e-99;
-    double zr, ze, dv;
-    // the three quotients in straight-line code, where the kernel gains from
-    // it, or with the operators (also where an operand is out of the range of
-    // ieee_div.cuh)
-    bool ops = true;
     if constexpr (kStraight) {
+        // the three quotients in straight-line code, or with the operators
+        // where an operand is out of its range (ieee_div.cuh)
         ieee::Guard g;
-        zr = ieee::quot(zm, zvol, ieee::rcp(zvol, g), g);
-        ze = ieee::quot0(zetot, zme, ieee::rcp(zme, g), g);
-        dv = ieee::quot0(dvol, zvol0, ieee::rcp(zvol0, g), g);
-        ops = !g.ok();
+        const double zme = zm + 1.e-99;
+        double zr = ieee::quot(zm, zvol, ieee::rcp(zvol, g), g);
+        double ze = ieee::quot0(zetot, zme, ieee::rcp(zme, g), g);
+        double dv = ieee::quot0(dvol, zvol0, ieee::rcp(zvol0, g), g);
+        if (!g.ok()) {
+            zr = zm / zvol;
+            ze = zetot / zme;
+            dv = dvol / zvol0;
+        }
+        a.zvol[z] = zvol;
+        a.zr[z] = zr;
+        a.zetot[z] = zetot;
+        a.ze[z] = ze;
+        a.zwrate[z] = zwrate;
+        return fabs(dv);
+    } else {
+        a.zvol[z] = zvol;
+        a.zr[z] = zm / zvol;
+        a.zetot[z] = zetot;
+        a.ze[z] = zetot / (zm + 1.e-99);
+        a.zwrate[z] = zwrate;
+        return fabs((zvol - zvol0) / zvol0);
     }
-    if (ops) {
-        zr = zm / zvol;
-        ze = zetot / zme;
-        dv = dvol / zvol0;
-    }
-    a.zvol[z] = zvol;
-    a.zr[z] = zr;
-    a.zetot[z] = zetot;
-    a.ze[z] = ze;
-    a.zwrate[z] = zwrate;
-    return fabs(dv);
 }
 
 // One zone's corrector from its inputs, read through `in` where they are
 // used: for side k < n, in.x(k) / in.u(k) the new position and velocity of
 // the side's first point, in.u0(k) its start-of-cycle velocity (before the
 // boundary projections), in.x0x(k) its start-of-cycle x, in.mask(k) its BC
-// plane mask (asked for where in.bc()), in.sf(k) the side's sfp + sfq; in.zm() etc. the zone's
+// plane mask, in.sf(k) the side's sfp + sfq; in.zm() etc. the zone's
 // scalars.  Writes zvol, zr, zetot, ze, zwrate; returns |dV/V0| and adds the
 // zone's inverted sides to nbad.
 template <bool kQuads, bool kMixed, typename In>
@@ -149,7 +152,6 @@ __device__ __forceinline__ double zone_core(const DevArrays& a, const HydroConst
     if (kQuads) n = 4;
     const double zm = in.zm(), zetot0 = in.zetot(), zvol0 = in.zvol(), zp = in.zp();
     const double dth = 0.5 * dt;
-    const bool bc = in.bc();
 
     double2 x[4], ub[4];
     double xpx[4];
@@ -160,7 +162,7 @@ __device__ __forceinline__ double zone_core(const DevArrays& a, const HydroConst
             const double2 u0 = in.u0(k);
             xpx[k] = in.x0x(k) + u0.x * dth;   // advPosHalf's x, from pu0 before the BCs
             // applyFixedBC on pu0 (Hydro.cc:1008-1032), planes in deck order
-            const unsigned mask = bc ? in.mask(k) : 0u;
+            const unsigned mask = in.mask(k);
             double2 u0b = u0;
             if (mask) {
                 for (int b = 0; b < c.nbc; ++b)
@@ -239,7 +241,6 @@ struct StagedIn {
         return reinterpret_cast<const double*>(st + kOffX0x)[k * kTile + t];
     }
     __device__ __forceinline__ double2 sf(int k) const { return sfg[k]; }
-    __device__ __forceinline__ bool bc() const { return true; }
     __device__ __forceinline__ unsigned mask(int k) const {
         const uint32_t w = reinterpret_cast<const uint32_t*>(st + kOffMw)[k * kTile + t];
         return (w >> (((meta >> (4 + k)) & 1) * 16)) & 0xffffu;
