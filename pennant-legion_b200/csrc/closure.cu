@@ -458,7 +458,8 @@ struct pnt_closure {
     uint8_t* d_trimg = nullptr;
     float* d_partial = nullptr;
     int partial_cap = 0;
-    float* d_loss = nullptr;     // [2]: loss, error flag
+    static constexpr int kLosses = 4096;
+    float* d_loss = nullptr;     // [kLosses]: losses of the steps since the host last read them
     float* d_grad = nullptr;
     int* d_err = nullptr;        // set by a training step whose tensor-core wait ran out
     int64_t adam_t = 0;
@@ -494,7 +495,7 @@ struct pnt_closure {
         CUDA_TRY(cudaMalloc(&d_trimg, train::kImgBytes));
         CUDA_TRY(cudaMalloc(&d_err, sizeof(int)));
         CUDA_TRY(cudaMemset(d_err, 0, sizeof(int)));
-        CUDA_TRY(cudaMalloc(&d_loss, 16));
+        CUDA_TRY(cudaMalloc(&d_loss, kLosses * sizeof(float)));
         CUDA_TRY(cudaMalloc(&d_grad, kClParams * sizeof(float)));
         CUDA_TRY(cudaMemset(d_img, 0, kImgBytes));
         CUDA_TRY(cudaMemset(d_trimg, 0, train::kImgBytes));
@@ -545,9 +546,10 @@ struct pnt_closure {
         partial_cap = nparts;
         return PNT_OK;
     }
-    // One gradient pass over rows (first + i) mod n, i < rows; Adam step when apply.
+    // One gradient pass over rows (first + i) mod n, i < rows; Adam step when
+    // apply.  The loss goes to d_loss[slot].
     pnt_status step(const void* x, const float* t, int64_t n, int64_t first, int64_t rows, float lr, bool apply,
-                    float* grad_host, float* loss_host) {
+                    float* grad_host, float* loss_host, int slot = 0) {
         const int nparts = (int)((rows + train::kRows - 1) / train::kRows);
         pnt_status st = ensure_partial(nparts);
         if (st) return st;
@@ -563,7 +565,7 @@ struct pnt_closure {
         }
         closure_reduce_adam<<<(kClParams + 1 + 31) / 32, kReduceThreads, 0, stream>>>(
             d_params, d_m, d_v, d_partial, nparts, lr, bc1, bc2, A.inv_count, apply ? 1 : 0,
-            grad_host ? d_grad : nullptr, d_loss);
+            grad_host ? d_grad : nullptr, d_loss + slot);
         CUDA_TRY(cudaGetLastError());
         if (apply) {
             pack_images<<<32, 256, 0, stream>>>(d_params, norm(), thr[0], thr[1], thr[2], d_img, d_trimg);
@@ -571,7 +573,7 @@ struct pnt_closure {
         }
         if (grad_host)
             CUDA_TRY(cudaMemcpyAsync(grad_host, d_grad, kClParams * sizeof(float), cudaMemcpyDeviceToHost, stream));
-        if (loss_host) CUDA_TRY(cudaMemcpyAsync(loss_host, d_loss, sizeof(float), cudaMemcpyDeviceToHost, stream));
+        if (loss_host) CUDA_TRY(cudaMemcpyAsync(loss_host, d_loss + slot, sizeof(float), cudaMemcpyDeviceToHost, stream));
         if (grad_host || loss_host) CUDA_TRY(cudaStreamSynchronize(stream));
         return PNT_OK;
     }
@@ -744,10 +746,20 @@ pnt_status pnt_closure_train(pnt_closure* c, const void* x, const float* t, int6
     if (!c || !x || !t || n <= 0 || first < 0 || steps < 0 || rows_per_step <= 0 || !(lr > 0.f))
         return fail(PNT_ERR_INVALID_ARG, "bad argument");
     DeviceGuard dg(c->device);
+    // the steps follow one another on the stream; the host reads their losses
+    // when the array is full and at the end (a read and a wait a step left the
+    // GPU idle for a launch latency a step)
+    constexpr int kCap = pnt_closure::kLosses;
     for (int s = 0; s < steps; ++s) {
         const int64_t f0 = (first + (int64_t)s * rows_per_step) % n;
-        pnt_status st = c->step(x, t, n, f0, rows_per_step, lr, true, nullptr, losses ? losses + s : nullptr);
+        const int slot = s % kCap;
+        pnt_status st = c->step(x, t, n, f0, rows_per_step, lr, true, nullptr, nullptr, slot);
         if (st) return st;
+        if (losses && (slot == kCap - 1 || s == steps - 1)) {
+            CUDA_TRY(cudaMemcpyAsync(losses + (s - slot), c->d_loss, (slot + 1) * sizeof(float), cudaMemcpyDeviceToHost,
+                                     c->stream));
+            CUDA_TRY(cudaStreamSynchronize(c->stream));
+        }
     }
     CUDA_TRY(cudaStreamSynchronize(c->stream));
     if (pnt_status st = c->check_err()) return st;

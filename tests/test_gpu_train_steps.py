@@ -1,0 +1,44 @@
+"""Closure training where its kernels' steps end: partial counts around the
+reduction's eight threads a parameter, and more steps than the losses' array
+on the device holds (4096)."""
+import numpy as np
+import pytest
+import torch
+
+import closure_oracle as co
+import pennant_b200 as pb
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def rows(n, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    x = torch.randn(n, 16, generator=g, device=DEV)
+    x[:, 14:] = 0
+    t = torch.randn(n, 4, generator=g, device=DEV)
+    torch.cuda.synchronize()
+    return x.bfloat16().contiguous(), t.contiguous()
+
+
+@pytest.mark.parametrize("n", [7 * 128, 8 * 128 + 1, 17 * 128, 32 * 128 + 5])
+def test_gradient_over_many_partials(n):
+    c = pb.Closure(seed=2)
+    x, t = rows(n, n)
+    torch.cuda.synchronize()
+    g, loss = c.gradient(x.data_ptr(), t.data_ptr(), n)
+    lo, go = co.loss_grad(c.get()[0], x[:, :14].float().cpu().numpy(), t.cpu().numpy(), bf16_round=True)
+    # the bounds of the gradient test at 128 to 1024 rows: the same rounding points a row
+    assert abs(loss - lo) <= 1e-4 * lo
+    for a, b in ((co.W1, co.B1), (co.B1, co.W2), (co.W2, co.B2), (co.B2, co.W3), (co.W3, co.B3), (co.B3, co.N_PARAMS)):
+        assert np.linalg.norm(g[a:b] - go[a:b]) < 2e-3 * np.linalg.norm(go[a:b]), (a, b)
+
+
+def test_losses_past_the_device_array():
+    x, t = rows(512, 1)
+    one, two = pb.Closure(seed=3), pb.Closure(seed=3)
+    a = one.train(x.data_ptr(), t.data_ptr(), 512, 0, 4098, 128, 1e-3)
+    b = [two.train(x.data_ptr(), t.data_ptr(), 512, (f * 128) % 512, k, 128, 1e-3) for f, k in ((0, 4095), (4095, 2), (4097, 1))]
+    assert np.array_equal(a, np.concatenate(b))
+    assert np.array_equal(one.get()[0], two.get()[0])
