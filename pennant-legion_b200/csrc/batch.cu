@@ -329,6 +329,7 @@ struct pnt_batch {
         if (nzt) CUDA_TRY(cudaMemcpy(ztiles, zt.data(), nzt * sizeof(Tile), cudaMemcpyHostToDevice));
         if (!pt.empty()) CUDA_TRY(cudaMemcpy(ptiles, pt.data(), pt.size() * sizeof(Tile), cudaMemcpyHostToDevice));
         CUDA_TRY(cudaMemcpy(inst_tbeg, tb.data(), tb.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaStreamSynchronize(nullptr));
         b.ztiles = ztiles;
         b.ptiles = ptiles;
         b.nztiles = (int32_t)nzt;
@@ -668,6 +669,11 @@ pnt_status pnt_batch_create(const pnt_mesh* const* meshes, const pnt_params* par
         if (e != cudaSuccess) {
             delete bt;
             return fail(PNT_ERR_CUDA, "batch setup: %s", cudaGetErrorString(e));
+        }
+        // the batch's stream does not wait for the default stream
+        if (cudaStreamSynchronize(nullptr) != cudaSuccess) {
+            delete bt;
+            return fail(PNT_ERR_CUDA, "batch setup: the uploads failed");
         }
         std::memcpy(bt->ctl_host, ctls.data(), sizeof(Ctl) * n);
         if ((st = bt->build_tiles(Shape{256, 3}))) {

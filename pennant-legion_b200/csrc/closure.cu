@@ -486,6 +486,8 @@ struct pnt_closure {
         return n;
     }
 
+    // Everything on the object's stream, which does not wait for the default
+    // stream: a memset there could still run after the images were packed.
     pnt_status setup() {
         CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         CUDA_TRY(cudaMalloc(&d_params, kClParams * sizeof(float)));
@@ -494,13 +496,13 @@ struct pnt_closure {
         CUDA_TRY(cudaMalloc(&d_img, kImgBytes));
         CUDA_TRY(cudaMalloc(&d_trimg, train::kImgBytes));
         CUDA_TRY(cudaMalloc(&d_err, sizeof(int)));
-        CUDA_TRY(cudaMemset(d_err, 0, sizeof(int)));
+        CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), stream));
         CUDA_TRY(cudaMalloc(&d_loss, kLosses * sizeof(float)));
         CUDA_TRY(cudaMalloc(&d_grad, kClParams * sizeof(float)));
-        CUDA_TRY(cudaMemset(d_img, 0, kImgBytes));
-        CUDA_TRY(cudaMemset(d_trimg, 0, train::kImgBytes));
-        CUDA_TRY(cudaMemset(d_m, 0, kClParams * sizeof(float)));
-        CUDA_TRY(cudaMemset(d_v, 0, kClParams * sizeof(float)));
+        CUDA_TRY(cudaMemsetAsync(d_img, 0, kImgBytes, stream));
+        CUDA_TRY(cudaMemsetAsync(d_trimg, 0, train::kImgBytes, stream));
+        CUDA_TRY(cudaMemsetAsync(d_m, 0, kClParams * sizeof(float), stream));
+        CUDA_TRY(cudaMemsetAsync(d_v, 0, kClParams * sizeof(float), stream));
         static bool attr_done[64] = {};
         if (device < 64 && !attr_done[device]) {
             CUDA_TRY(cudaFuncSetAttribute(train::grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -458,7 +458,7 @@ pnt_status pnt_hydro_create(const pnt_mesh* mesh, const pnt_params* params, int3
         if (!st && h->learned) {
             unsigned long long* counts = nullptr;
             st = h->alloc(&counts, kClassCount * 64);
-            if (!st && cudaMemset(counts, 0, kClassCount * 64 * sizeof(unsigned long long)) != cudaSuccess)
+            if (!st && cudaMemsetAsync(counts, 0, kClassCount * 64 * sizeof(unsigned long long), h->stream) != cudaSuccess)
                 st = fail(PNT_ERR_CUDA, "counter memset failed");
             h->a.closure_counts = counts;
         }
