@@ -56,19 +56,18 @@ DEFAULT_DECK = os.path.join(PKG, "decks", "sedov1920.pnt")
 DEFAULT_CLOSURE = os.path.join(PKG, "closure", "qcs_mlp.bin")
 MLP_FLOP_PER_ROW = 2 * (16 * 64 + 64 * 64 + 64 * 16)   # tensor-core MMA shapes, padded
 # DRAM bytes (read + write) of one pass A launch per zone, from the ncu
-# captures of profiles/pass_a_rows_learned_sedov1024.md (learned, mixed)
-# and profiles/pass_a_fp64_sedov1024.md (FP64), 1,048,576 zones each; the
-# bench scales them by its zone count
-PASS_A_TRAFFIC_PER_ZONE = {"learned": (109.723e6 + 81.982e6) / 1048576,
-                           "mixed": (109.362e6 + 76.070e6) / 1048576,
-                           "fp64": (125.973e6 + 130.137e6) / 1048576}
+# captures of profiles/pass_a_warp_stages_sedov1024.md, 1,048,576 zones
+# each; the bench scales them by its zone count
+PASS_A_TRAFFIC_PER_ZONE = {"learned": (111.112e6 + 77.292e6) / 1048576,
+                           "mixed": (111.099e6 + 78.807e6) / 1048576,
+                           "fp64": (109.265e6 + 121.266e6) / 1048576}
 
 
 # FP64 thread-instructions a zone of one FP64 pass A launch (ncu
-# sm__sass_thread_inst_executed_op_fp64_pred_on, 1024^2 Sedov at cycle
-# 16000: profiles/pass_a_fp64_sedov1024.md), and the B200's FP64 rate a
+# sm__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on, 1024^2 Sedov:
+# profiles/pass_a_warp_stages_sedov1024.md), and the B200's FP64 rate a
 # clock per SM (sm__sass_thread_inst_executed_op_dfma_pred_on peak)
-FP64_PASS_A_INST_PER_ZONE = 907.6
+FP64_PASS_A_INST_PER_ZONE = 713.6
 FP64_INST_PER_CLOCK_PER_SM = 64
 
 
@@ -770,7 +769,7 @@ def main():
         ach = FP64_PASS_A_INST_PER_ZONE * nz / (ms / 1e3) / 1e12
         return {"bound": "fp64 pipe", "kernel": "pass A (fp64)", "achieved": ach, "peak": peak,
                 "unit": "T FP64 thread-instructions/s", "frac": ach / peak, "launch_ms": ms,
-                "note": "FP64 instructions a zone from profiles/pass_a_fp64_sedov1024.md (1024^2 at cycle "
+                "note": "FP64 instructions a zone from profiles/pass_a_warp_stages_sedov1024.md (1024^2 at cycle "
                         "16000); the count depends on how much of the mesh is quiescent"}
 
     kms_head = res[args.precision]["kernel_ms"]
