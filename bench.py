@@ -831,7 +831,7 @@ def main():
                          "peak": hbm, "unit": "GB/s", "frac": ach_dom / hbm, "peak_kind": peak_kind,
                          "algorithmic_bytes_per_launch": per_launch[names[dom]], "launch_ms": kms_head[dom],
                          "traffic": PASS_A_TRAFFIC_PER_ZONE[args.precision] * numz if names[dom] == "A" else None,
-                         "traffic_note": "ncu DRAM read+write of one pass A launch at 1024^2 (cycle 16000), "
+                         "traffic_note": "ncu DRAM read+write of one pass A launch at 1024^2, "
                                          "scaled by the zone count (writes still in L2 at the kernel's end "
                                          "are not counted)"},
             "roofline_fp64_pass_a": fp64_pipe_roofline(res["fp64"]["kernel_ms"][0], numz),
