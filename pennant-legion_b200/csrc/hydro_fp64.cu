@@ -117,9 +117,7 @@ __global__ void __launch_bounds__(kSmallThreads) pass_a_small(DevArrays a, Hydro
         kKind == kRect ? zstage::rect_idx(z, a.rect_nzx, 0, 0) : zstage::load_idx(a, z, kKind == kQuads);
     double zdthyd = 1.e99;
     int bad = 0;
-    const bool ok = pass_a_zone_lanes(a, c, cur, dt, z, ix.s0, ix.n, ix.p, live, zdthyd, bad);
-    const unsigned m = __ballot_sync(kFull, !ok) >> (lane & ~3);
-    if (m & 0xfu) {
+    if (!pass_a_zone_lanes(a, c, cur, dt, z, ix.s0, ix.n, ix.p, live, zdthyd, bad)) {
         zdthyd = 1.e99;
         bad = 0;
         if (live && (lane & 3) == 0) {

@@ -595,9 +595,11 @@ __device__ __forceinline__ bool pass_a_zone_fast(const DevArrays& a, const Hydro
 // thread leaves most schedulers without a warp, where the time is one warp's
 // way through the code.  Zone quantities are formed in every lane, sums over
 // the sides in side order through shuffles, so the bits are those of
-// pass_a_zone_fast.  ix: the zone's points; a lane without a zone calls it
-// too (live = false, on any valid zone) and stores nothing.  Returns whether
-// the lane's operands were in range; the zone stands when all four lanes' were.
+// pass_a_zone_fast.  p: the zone's points; a lane without a zone calls it
+// too (live = false, on any valid zone) and stores nothing.  Returns, the same
+// in its four lanes, whether all their operands were in range; a zone with one
+// that was not is not stored either, so that the lane that forms it again is
+// the only one that writes it.
 // ---------------------------------------------------------------------
 __device__ __forceinline__ bool pass_a_zone_lanes(const DevArrays& a, const HydroConst& c, int cur, double dt,
                                                   int32_t z, int32_t s0, int n, const int32_t* p, bool live,
@@ -714,13 +716,14 @@ __device__ __forceinline__ bool pass_a_zone_lanes(const DevArrays& a, const Hydr
     const double2 sfpq = add(smul(-zp, ssurf), mk(fs.x * rinv, fs.y * rinv));
     const double2 ftot = add(sfpq, smul(-sdp, ssurf));
     const double2 fv = shfl2(ftot, lp);
-    if (mine) {
+    const bool stands = ((__ballot_sync(kFull, !(g.ok() && still)) >> gl) & 0xfu) == 0;
+    if (mine && stands) {
         a.cmass[s0 + k] = cm;
         a.sftot[s0 + k] = sfpq;
         a.cforce[s0 + k] = sub(ftot, fv);
         if (k == 0) a.zp[z] = zp;
     }
-    return g.ok() && still;
+    return stands;
 }
 
 // ---------------------------------------------------------------------
