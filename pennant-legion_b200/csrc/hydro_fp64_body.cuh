@@ -400,7 +400,9 @@ __device__ __forceinline__ void pass_a_zone_thread(const DevArrays& a, const Hyd
 // as small as they are it is not refused:
 //  - q and the velocity differences over the edges enter sums with, or are
 //    compared with, the sound speed, which is at least 1e-50: below that they
-//    need not be exact (quot_unchecked);
+//    need not be exact (quot_unchecked); too large a dividend is refused all
+//    the same (an infinite quotient would come out as a NaN, which the maxima
+//    drop, and hide a run that blew up from dt);
 //  - zkur adds du to the sound speed's term; where that is 2^-200 or more,
 //    a du below 2^-400 does not change it;
 //  - only the sign of the reference's cdiv is used: that of its dividend times
@@ -454,6 +456,7 @@ __device__ __forceinline__ bool pass_a_zone_fast(const DevArrays& a, const Hydro
         rinv[k] = ieee::rcp(elen[k], g);
         zdl = dmin(zdl, ieee::quot(fac * sa[k], elen[k], rinv[k], g));
         const double dux = dot(sub(u0[nk], u0[k]), dxs);
+        g.below(dux);
         dumax = dmax(dumax, ieee::quot_unchecked(fabs(dux), elen[k], rinv[k]));
     }
     // PolyGas::calcStateHalf with calcRho
@@ -461,6 +464,7 @@ __device__ __forceinline__ bool pass_a_zone_fast(const DevArrays& a, const Hydro
     const double p = c.gm1 * zr * e;
     const double pre = c.gm1 * e;
     const double per = c.gm1 * zr;
+    g.below(per * p);
     const double q = ieee::quot_unchecked(per * p, zr * zr, ieee::rcp(zr * zr, g));
     const double minv = ieee::rcp(zm, g);
     const double csqd = dmax(c.ssmin2, pre + q);
@@ -630,7 +634,9 @@ __device__ __forceinline__ bool pass_a_zone_lanes(const DevArrays& a, const Hydr
     const double rinv = ieee::rcp(elen, g);
     const double elenv = shfl(elen, lp), rinvv = shfl(rinv, lp);
     double zdl = dmin(1.e99, ieee::quot(fac * sa, elen, rinv, g));
-    double dumax = dmax(0., ieee::quot_unchecked(fabs(dot(sub(un, u), dxs)), elen, rinv));
+    const double dux = dot(sub(un, u), dxs);
+    g.below(dux);
+    double dumax = dmax(0., ieee::quot_unchecked(fabs(dux), elen, rinv));
 #pragma unroll
     for (int o = 1; o < 4; o <<= 1) {   // an idle lane holds side 0's
         zdl = dmin(zdl, __shfl_xor_sync(kFull, zdl, o));
@@ -641,6 +647,7 @@ __device__ __forceinline__ bool pass_a_zone_lanes(const DevArrays& a, const Hydr
     const double pr = c.gm1 * zr * e;
     const double pre = c.gm1 * e;
     const double per = c.gm1 * zr;
+    g.below(per * pr);
     const double qe = ieee::quot_unchecked(per * pr, zr * zr, ieee::rcp(zr * zr, g));
     const double minv = ieee::rcp(zm, g);
     const double csqd = dmax(c.ssmin2, pre + qe);

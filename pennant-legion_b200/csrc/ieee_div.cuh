@@ -7,7 +7,9 @@
 // results are formed in straight-line code, which the compiler interleaves,
 // quotients over one divisor share its reciprocal, and every operand's
 // range goes into a Guard that the caller tests once: a zone with any
-// operand out of range is formed again with the operators.
+// operand out of range is formed again with the operators.  Only the
+// dividends of quot_unchecked are the caller's to check: against their upper
+// limit (Guard::below), and for what too small a one does to its result.
 //
 // Quotients (P. Markstein, IBM J. Res. Dev. 34 (1990) 111; M. Cornea, J.
 // Harrison, P. Tang, "Scientific Computing on Itanium-based Systems", 2002).
@@ -70,7 +72,7 @@ __device__ __forceinline__ double rcp(double b, Guard& g) {
     return (ones == 0xffffffffu) ? __hiloint2double(__double2hiint(y), 1) : y;
 }
 // a / b from y = rcp(b) for a in range or +0; smaller a give some value
-// below 2^-499.
+// below 2^-499.  For |a| of 2^300 or more (Guard::below) it may be a NaN.
 __device__ __forceinline__ double quot_unchecked(double a, double b, double y) {
     const double q0 = __dmul_rn(a, y);
     return __fma_rn(__fma_rn(-b, q0, a), y, q0);
