@@ -406,8 +406,8 @@ __device__ __forceinline__ void pass_a_zone_thread(const DevArrays& a, const Hyd
 //  - zkur adds du to the sound speed's term; where that is 2^-200 or more,
 //    a du below 2^-400 does not change it;
 //  - only the sign of the reference's cdiv is used: that of its dividend times
-//    that of its divisor, unless the quotient underflows, which it cannot
-//    over a divisor up to 1 (every edge below 1/2).
+//    that of its divisor (infinities and NaN included), unless the quotient
+//    underflows, which it cannot over a divisor up to 1 (every edge below 1/2).
 // Other differences in form:
 //  - the corners' angles and weights are formed for all corners at once
 //    (their quotients interleave), and the side forces at the end from the
@@ -514,7 +514,6 @@ __device__ __forceinline__ bool pass_a_zone_fast(const DevArrays& a, const Hydro
         cc[k] = flat ? 0. : ccos;
         const double num = cross(sub(zuc, u), d31) - cross(sub(up3, up1), d20);
         g.divisor(2.0 * cvolume);
-        g.below(num);
         sdiv[k] = (cvolume < 0.0) ? -num : num;
     }
     double emax = elen[0];
@@ -684,7 +683,6 @@ __device__ __forceinline__ bool pass_a_zone_lanes(const DevArrays& a, const Hydr
     const double cc = flat ? 0. : ccos;
     const double num = cross(sub(zuc, u), d31) - cross(sub(up3, up1), d20);
     g.divisor(2.0 * cvolume);
-    g.below(num);
     g.dividend((fabs(cvolume) > 0.5 && num != 0.0) ? num : 1.0);
     const double sdiv = (cvolume < 0.0) ? -num : num;
     const double ztmp1 = c.q1 * zss;

@@ -81,3 +81,15 @@ def test_edge_velocity_that_overflows_without_divergence(n):
         return {"pu": o.field("px") * np.array([1.0, -1.0]) * 2.0 ** (1024 - 66)}
     s = check_one_cycle(text, change)
     assert s["dtnew"] == 0.0
+
+
+@pytest.mark.parametrize("n", [8, 136])
+def test_divergence_that_is_no_number(n):
+    # u = A (-y, x): the edges' (du . dx) are zeros, and the divergence is
+    # the difference of two products A h^2 / 4 that overflow
+    h = 2.0 ** 33
+    text = deck_text(("rect", n, n), lx=n * h, dtinit=1e-307)
+
+    def change(o):
+        return {"pu": o.field("px")[:, ::-1] * np.array([-1.0, 1.0]) * 2.0 ** (1024 - 64)}
+    check_one_cycle(text, change)
