@@ -298,12 +298,13 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
     int32_t *zfirst = nullptr, *znump = nullptr, *mapsp1 = nullptr, *poff = nullptr, *pcorner = nullptr;
     double* smf = nullptr;
     uint16_t* mask = nullptr;
-    uint8_t* zone_bc = nullptr;
+    uint16_t* zone_bc = nullptr;
     // the persistent pass C's grid
     {
         int nsm = 148;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-        cudaError_t e = prepare_pass_c(p.precision != PNT_PREC_FP64, a.quads != 0, a.rect_nzx, a.numz, nsm, &a.gridC);
+        cudaError_t e = prepare_pass_c(p.precision != PNT_PREC_FP64, a.quads != 0, a.rect_nzx, c.nbc, a.numz, nsm,
+                                       &a.gridC);
         if (e != cudaSuccess) return fail(PNT_ERR_CUDA, "pass C setup: %s", cudaGetErrorString(e));
         if (p.precision == PNT_PREC_FP64) {
             int32_t ntiles = 0;

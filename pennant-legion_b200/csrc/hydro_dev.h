@@ -99,7 +99,7 @@ struct DevArrays {
     // -dvovmax, inverted sides in A, in C] here instead of ending the cycle
     // (nullptr for a single piece)
     double* piece_red;
-    const uint8_t* zone_bc;   // [numz] the zone has a point on a BC plane (pass C on rect meshes)
+    const uint16_t* zone_bc;  // [numz] the BC plane masks of the zone's points in a word (pass C on rect meshes)
 };
 
 constexpr int kZoneThreads = 256;   // pass A: 64 zones x 4 side lanes per block
@@ -179,10 +179,11 @@ cudaError_t prepare_learned_kernels();
 // device and returns its persistent grid (resident CTAs per SM x nsm, at
 // most one per tile); launch_pass_c launches it with a.gridC CTAs, which
 // write a.gridC partials.
-cudaError_t prepare_pass_c(bool mixed, bool quads, int32_t rect_nzx, int32_t numz, int nsm, int32_t* grid);
+cudaError_t prepare_pass_c(bool mixed, bool quads, int32_t rect_nzx, int32_t nbc, int32_t numz, int nsm,
+                           int32_t* grid);
 void launch_pass_c(const DevArrays& a, const HydroConst& c, bool mixed, cudaStream_t stream);
 // a.zone_bc from the mesh and the points' masks (pass_c.cu).
-cudaError_t launch_find_zone_bc(const DevArrays& a, uint8_t* zone_bc, cudaStream_t stream);
+cudaError_t launch_find_zone_bc(const DevArrays& a, uint16_t* zone_bc, cudaStream_t stream);
 // Pass A of the FP64 cycle (hydro_fp64.cu) and of the mixed or learned cycle
 // (hydro_mixed.cu): raises the kernel's shared-memory limit on the current
 // device and returns its persistent grid (and the tiles a.redo holds a word

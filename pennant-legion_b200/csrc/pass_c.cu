@@ -19,13 +19,18 @@ namespace {
 // Pass C over row tiles of a rect mesh (row_tiles.cuh): per tile of up to
 // kRowT zones, the bottom and top point rows of px0, pu0, px, pu and four
 // zone fields arrive by bulk copies; each thread reads its zone's sfp + sfq
-// (64 contiguous bytes) from global memory, and the BC plane masks where its
-// zone has a point on a plane (a flag a zone, read a tile ahead: the masks of
-// every zone were a second memory latency a tile).  64 zones and two stages a
-// CTA, shared memory for 10 CTAs an SM.  Bound by latency and HBM: 1920^2
-// Sedov 0.135 ms (its 190 bytes a zone take 0.107 ms); 0.146 ms with the masks
-// of every zone and the division operator, 0.150 ms without the prefetch of
-// sfp + sfq into L2 too; that one against 0.163 ms with sfp + sfq in the stages
+// (64 contiguous bytes) from global memory, and the BC plane masks of its four
+// points as one word of four bits a point, a tile ahead (the masks point by
+// point were a second memory latency a tile; a flag a zone with the masks
+// behind it, the same latency again in every tile of a boundary row or
+// column).  64 zones and two stages a CTA, shared memory for 10 CTAs an SM.
+// Bound by latency and HBM: 1920^2 Sedov 0.126 ms (its 190 bytes a zone take
+// 0.107 ms); 0.135 ms with the flag, 0.134 ms with the masks of every zone,
+// 0.146 ms with those and the division operator, 0.150 ms without the prefetch
+// of sfp + sfq into L2 too; 480^2 Noh 17.8 us, 20.2 with the flag, 19.5 with
+// the masks, 19.0 with those and neither prefetch nor straight-line quotients
+// (Sedov, whose zones at rest divide zeros: 18.1, 20.2, 19.5, 20.3).  The
+// 0.150 ms against 0.163 ms with sfp + sfq in the stages
 // (7 CTAs an SM), 0.152 ms with the zone fields also from global memory,
 // 0.174-0.185 ms with three stages or sfp + sfq held a tile ahead in registers
 // (8 CTAs) and 0.173 ms for the staged gathers.
@@ -50,6 +55,11 @@ static_assert(kRowT % 2 == 0 && kRowStageBytes % 16 == 0, "16-byte aligned stage
 // stay, the prefetch cost 2%).
 constexpr int32_t kPrefetchZones = 500000;
 
+constexpr int kWordPlanes = 4;   // planes of a zone's word: bits a point
+
+// kFew: at most kWordPlanes planes, the masks of the zone's points in a word.
+// Decks of more planes, which no case has, read them point by point.
+template <bool kFew>
 struct RowIn {
     static constexpr bool kStraight = true;
     const unsigned char* st;
@@ -67,9 +77,9 @@ struct RowIn {
     __device__ __forceinline__ double2 u(int k) const { return *f(3, k); }
     const double2* sfg;   // the zone's sfp + sfq (global memory)
     __device__ __forceinline__ double2 sf(int k) const { return sfg[k]; }
-    bool any_bc;          // a point of the zone is on a BC plane
+    unsigned word;
     __device__ __forceinline__ unsigned mask(int k) const {
-        return any_bc ? __ldg(bcmask + pb + row(k) * npx + col(k)) : 0u;
+        return kFew ? (word >> (kWordPlanes * k)) & ((1u << kWordPlanes) - 1u) : __ldg(bcmask + pb + row(k) * npx + col(k));
     }
     __device__ __forceinline__ double zs(int fld) const {
         return reinterpret_cast<const double*>(st + kRowOffZs + fld * kRowZB)[shift + t];
@@ -80,7 +90,7 @@ struct RowIn {
     __device__ __forceinline__ double zp() const { return zs(3); }
 };
 
-template <bool kMixed>
+template <bool kMixed, bool kFew>
 __global__ void __launch_bounds__(kRowT) pass_c_rows(DevArrays a, HydroConst c) {
     extern __shared__ __align__(128) unsigned char smem_r[];
     __shared__ __align__(8) uint64_t bars[kRowStages];
@@ -118,23 +128,23 @@ __global__ void __launch_bounds__(kRowT) pass_c_rows(DevArrays a, HydroConst c) 
         for (int f = 0; f < 4; ++f)
             rows::bulk_g2s(st + kRowOffZs + f * kRowZB, zf[f] + zr.zs, (uint32_t)(zr.count * 8), bar);
     };
-    // whether the thread's zone of tile g has a point on a BC plane, a tile
-    // ahead; and the next tile's sfp + sfq into L2
+    // the plane masks of the thread's zone of tile g, a tile ahead; and that
+    // tile's sfp + sfq into L2
     const bool far = a.numz > kPrefetchZones;
-    auto look_ahead = [&](int64_t g) -> uint8_t {
-        if (g >= ntiles) return 0;
+    auto look_ahead = [&](int64_t g) -> unsigned {
+        if (g >= ntiles || !(kFew || far)) return 0;
         const rows::Tile tn = rows::tile_of<kRowT>(g, nzx);
         if (t >= tn.nt) return 0;
         if (far) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.sftot + 4 * (tn.z0 + t)));
-        return __ldg(a.zone_bc + tn.z0 + t);
+        return kFew ? __ldg(a.zone_bc + tn.z0 + t) : 0u;
     };
-    uint8_t bc_next = look_ahead(blockIdx.x);
+    unsigned next_word = look_ahead(blockIdx.x);
     auto compute = [&](const unsigned char* st, int64_t g) {
         const rows::Tile tl = rows::tile_of<kRowT>(g, nzx);
-        const bool bc = bc_next != 0;
-        bc_next = look_ahead(g + gridDim.x);
+        const unsigned word = next_word;
+        next_word = look_ahead(g + gridDim.x);
         if (t >= tl.nt) return;
-        const RowIn in{st, a.bcmask, tl.pb, npx, t, (int)(tl.z0 & 1), a.sftot + 4 * (tl.z0 + t), bc};
+        const RowIn<kFew> in{st, a.bcmask, tl.pb, npx, t, (int)(tl.z0 & 1), a.sftot + 4 * (tl.z0 + t), word};
         const double d = stagedc::zone_core<true, kMixed>(a, c, 4, in, tl.z0 + t, dt, dtinv, nbad);
         dvm = (d > dvm) ? d : dvm;
     };
@@ -239,13 +249,14 @@ __global__ void __launch_bounds__(kSmallThreads) pass_c_small(DevArrays a, Hydro
     fp64::end_cycle_if_last(a, c);
 }
 
-// Which zones have a point on a BC plane.
-__global__ void find_zone_bc(DevArrays a, uint8_t* zone_bc) {
+// The BC plane masks of each zone's points in a word (not read where there are
+// more than kWordPlanes planes).
+__global__ void find_zone_bc(DevArrays a, uint16_t* zone_bc) {
     const int64_t z = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (z >= a.numz) return;
     unsigned m = 0;
-    for (int k = 0; k < a.znump[z]; ++k) m |= a.bcmask[a.mapsp1[a.zfirst[z] + k]];
-    zone_bc[z] = m ? 1 : 0;
+    for (int k = 0; k < a.znump[z]; ++k) m |= (unsigned)a.bcmask[a.mapsp1[a.zfirst[z] + k]] << (kWordPlanes * k);
+    zone_bc[z] = (uint16_t)m;
 }
 
 using Kernel = void (*)(DevArrays, HydroConst);
@@ -261,6 +272,11 @@ Kernel pick_small(int32_t rect_nzx, bool quads) {
                         : (quads ? pass_c_small<zstage::kQuads, kMixed> : pass_c_small<zstage::kGeneral, kMixed>);
 }
 
+Kernel pick_rows(bool mixed, bool few) {
+    if (mixed) return few ? pass_c_rows<true, true> : pass_c_rows<true, false>;
+    return few ? pass_c_rows<false, true> : pass_c_rows<false, false>;
+}
+
 Kernel pick_kernel(bool mixed, bool quads) {
     if (mixed) return quads ? pass_c_staged<true, true> : pass_c_staged<false, true>;
     return quads ? pass_c_staged<true, false> : pass_c_staged<false, false>;
@@ -268,13 +284,14 @@ Kernel pick_kernel(bool mixed, bool quads) {
 
 }  // namespace
 
-cudaError_t prepare_pass_c(bool mixed, bool quads, int32_t rect_nzx, int32_t numz, int nsm, int32_t* grid) {
+cudaError_t prepare_pass_c(bool mixed, bool quads, int32_t rect_nzx, int32_t nbc, int32_t numz, int nsm,
+                           int32_t* grid) {
     if (numz <= kSmallZones) {
         *grid = (numz + kSmallThreads / 4 - 1) / (kSmallThreads / 4);
         return cudaSuccess;
     }
     if (rect_nzx > 0) {
-        const Kernel k = mixed ? pass_c_rows<true> : pass_c_rows<false>;
+        const Kernel k = pick_rows(mixed, nbc <= kWordPlanes);
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowSmemBytes);
         if (e != cudaSuccess) return e;
         int occ = 0;
@@ -290,7 +307,7 @@ cudaError_t prepare_pass_c(bool mixed, bool quads, int32_t rect_nzx, int32_t num
     return tiles::prepare(pick_kernel(mixed, quads), stagedc::kTile, stagedc::kSmemBytes, numz, nsm, grid);
 }
 
-cudaError_t launch_find_zone_bc(const DevArrays& a, uint8_t* zone_bc, cudaStream_t stream) {
+cudaError_t launch_find_zone_bc(const DevArrays& a, uint16_t* zone_bc, cudaStream_t stream) {
     find_zone_bc<<<(unsigned)((a.numz + 255) / 256), 256, 0, stream>>>(a, zone_bc);
     return cudaGetLastError();
 }
@@ -302,7 +319,7 @@ void launch_pass_c(const DevArrays& a, const HydroConst& c, bool mixed, cudaStre
         return;
     }
     if (a.rect_nzx > 0) {
-        launch_pdl(mixed ? pass_c_rows<true> : pass_c_rows<false>, a.gridC, kRowT, kRowSmemBytes, stream, a, c);
+        launch_pdl(pick_rows(mixed, c.nbc <= kWordPlanes), a.gridC, kRowT, kRowSmemBytes, stream, a, c);
         return;
     }
     launch_pdl(pick_kernel(mixed, a.quads != 0), a.gridC, stagedc::kTile, stagedc::kSmemBytes, stream, a, c);

@@ -55,6 +55,15 @@ def test_no_linear_viscosity_and_planes_inside_the_mesh(nx, ny):
     check(deck_text(nx, ny, q1=0.0, planes=f"bcx 0.0 {1.0 / nx * (nx // 2)!r}\nbcy 0.0 {1.0 / nx * (ny // 3)!r}"))
 
 
+@pytest.mark.parametrize("nbcx,nbcy", [(0, 0), (2, 2), (4, 0), (3, 2), (9, 7)])
+def test_few_and_many_planes(nbcx, nbcy):
+    # 40090 zones: pass C's row tiles, whose words hold the masks of four planes
+    nx, ny = 211, 190
+    planes = "".join(f"{name} {' '.join(repr(1.0 / nx * (n * k // 10)) for k in range(count))}\n"
+                     for name, n, count in (("bcx", nx, nbcx), ("bcy", ny, nbcy)) if count)
+    check(deck_text(nx, ny, planes=planes.strip()))
+
+
 def test_batch_of_them_matches_single_runs():
     texts = [deck_text(9, 7), deck_text(9, 7, scale=1.0e25), deck_text(1, 1), deck_text(211, 190, scale=1.0e-24),
              deck_text(12, 9, mesh="pie"), deck_text(130, 127)]
