@@ -100,10 +100,12 @@ struct DevArrays {
     // (nullptr for a single piece)
     double* piece_red;
     const uint16_t* zone_bc;  // [numz] the BC plane masks of the zone's points in a word (pass C on rect meshes)
+    int32_t many;             // a point has more than kManyCorners corners
 };
 
 constexpr int kZoneThreads = 256;   // pass A: 64 zones x 4 side lanes per block
 constexpr int kPointThreads = 256;
+constexpr int kManyCorners = 8;     // pass B: points of more are gathered by their warp
 
 inline int64_t zone_blocks(int32_t numz, int threads = kZoneThreads) {
     return (4 * (int64_t)numz + threads - 1) / threads;

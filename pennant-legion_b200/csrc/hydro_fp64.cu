@@ -131,16 +131,16 @@ __global__ void __launch_bounds__(kSmallThreads) pass_a_small(DevArrays a, Hydro
     block_to_cycle<true, kSmallThreads>(a.cyc_red, zdthyd, nbad);
 }
 
-template <bool kRectPoints>
+template <PointKind kKind>
 __global__ void __launch_bounds__(kPointThreads) pass_b(DevArrays a, HydroConst c) {
     pdl_wait();
     const Ctl* ctl = a.ctl;
     if (skip_cycle(ctl)) return;
     const int64_t p = (int64_t)blockIdx.x * kPointThreads + threadIdx.x;
-    if (kRectPoints) {
+    if (kKind == kRectPoints) {
         if (p < a.nump) pass_b_point_rect<false>(a, c, ctl->cycle & 1, ctl->dt, p, a.rect_nzx, a.numz / a.rect_nzx);
     } else {
-        pass_b_point_csr<false>(a, c, ctl->cycle & 1, ctl->dt, p, p < a.nump);
+        pass_b_point_csr<false, kKind == kPointsOfMany>(a, c, ctl->cycle & 1, ctl->dt, p, p < a.nump);
     }
 }
 
@@ -209,7 +209,8 @@ cudaError_t launch_cycle_fp64(const DevArrays& a, const HydroConst& c, cudaStrea
     }
     if (phases & kPhaseAdvance) {
         const cudaError_t eb =
-            launch_pdl(a.rect_nzx > 0 ? pass_b<true> : pass_b<false>, pb, kPointThreads, 0, stream, a, c);
+            launch_pdl(a.rect_nzx > 0 ? pass_b<kRectPoints> : (a.many ? pass_b<kPointsOfMany> : pass_b<kPointsOfFew>), pb,
+                       kPointThreads, 0, stream, a, c);
         if (e == cudaSuccess) e = eb;
         if (ev) cudaEventRecord(ev[3], stream);
         launch_pass_c(a, c, false, stream);   // its last CTA ends the cycle

@@ -785,6 +785,10 @@ __device__ __forceinline__ int rect_point_corners(int32_t nzx, int32_t nzy, int6
     return n;
 }
 
+// How pass B finds a mesh's corners: from the point's index, or from the CSR
+// with or without points of more than kManyCorners corners.
+enum PointKind { kRectPoints, kPointsOfFew, kPointsOfMany };
+
 // A point's corner mass and force, FP64 cycle (mixed = false) or widened
 // from FP32.
 template <bool kMixed>
@@ -829,15 +833,17 @@ __device__ __forceinline__ void pass_b_point_rect(const DevArrays& a, const Hydr
 }
 
 // A point of any mesh through the point-to-corner CSR; called by whole warps
-// (live = false: no point).  A point of many corners, as the origin of a pie
+// (live = false: no point).  kMany (DevArrays::many): the mesh has points of
+// more than kManyCorners corners.  Such a point, as the origin of a pie
 // mesh (as many as its triangles), would keep its thread for a gather latency
 // every few corners, 0.2 us a corner; so from 9 corners on (two of the
 // single thread's gather steps) the warp gathers them 32 at a time and three
 // lanes add mass and force in order from shared memory.  Pass B of a 313 x
 // 801 pie: 68 -> 18.6 us, of a 200 x 200 one 21.0 -> 10.6 us (3 us of each
 // the launch); what is left of the origin is the chain of its additions.
-constexpr int kManyCorners = 8;
-template <bool kMixed>
+// Without such points the warp's part is left out: with it the mixed pass B
+// of a quad mesh of 1024^2 took 32.4 against 31.0 us, of 480^2 10.8 / 10.6.
+template <bool kMixed, bool kMany>
 __device__ __forceinline__ void pass_b_point_csr(const DevArrays& a, const HydroConst& c, int cur, double dt,
                                                  int64_t p, bool live) {
     int32_t o0 = 0, o1 = 0;
@@ -850,7 +856,7 @@ __device__ __forceinline__ void pass_b_point_csr(const DevArrays& a, const Hydro
     }
     double m = 0.;
     double2 f = mk(0., 0.);
-    const bool many = o1 - o0 > kManyCorners;
+    const bool many = kMany && o1 - o0 > kManyCorners;
     if (!many) {
         for (int32_t i = o0; i < o1; ++i) {
             double cm;
@@ -860,32 +866,34 @@ __device__ __forceinline__ void pass_b_point_csr(const DevArrays& a, const Hydro
             f = mk(__dadd_rn(f.x, cf.x), __dadd_rn(f.y, cf.y));
         }
     }
-    const int lane = threadIdx.x & 31;
-    for (unsigned left = __ballot_sync(kFull, many); left; left &= left - 1) {
-        __shared__ double vals[kPointThreads / 32][3][32];   // mass, force x, force y of 32 corners
-        double(*v)[32] = vals[threadIdx.x >> 5];
-        const int who = __ffs(left) - 1;
-        const int32_t b = __shfl_sync(kFull, o0, who), e = __shfl_sync(kFull, o1, who);
-        const double* mine = v[min(lane, 2)];   // lanes 0, 1, 2 add one component each
-        double sum = 0., cm = 0.;
-        double2 cf = mk(0., 0.);
-        if (b + lane < e) corner_values<kMixed>(a, __ldg(a.pcorner + b + lane), cm, cf);
-        for (int32_t i = b; i < e; i += 32) {
-            v[0][lane] = cm;   // +0 past the last corner, which leaves the sums as they are
-            v[1][lane] = cf.x;
-            v[2][lane] = cf.y;
-            __syncwarp();
-            cm = 0.;
-            cf = mk(0., 0.);
-            if (i + 32 + lane < e) corner_values<kMixed>(a, __ldg(a.pcorner + i + 32 + lane), cm, cf);
-#pragma unroll
-            for (int q = 0; q < 32; ++q) sum = __dadd_rn(sum, mine[q]);
-            __syncwarp();
-        }
-        const double wm = shfl(sum, 0), wx = shfl(sum, 1), wy = shfl(sum, 2);
-        if (lane == who) {
-            m = wm;
-            f = mk(wx, wy);
+    if constexpr (kMany) {
+        const int lane = threadIdx.x & 31;
+        for (unsigned left = __ballot_sync(kFull, many); left; left &= left - 1) {
+            __shared__ double vals[kPointThreads / 32][3][32];   // mass, force x, force y of 32 corners
+            double(*v)[32] = vals[threadIdx.x >> 5];
+            const int who = __ffs(left) - 1;
+            const int32_t b = __shfl_sync(kFull, o0, who), e = __shfl_sync(kFull, o1, who);
+            const double* mine = v[min(lane, 2)];   // lanes 0, 1, 2 add one component each
+            double sum = 0., cm = 0.;
+            double2 cf = mk(0., 0.);
+            if (b + lane < e) corner_values<kMixed>(a, __ldg(a.pcorner + b + lane), cm, cf);
+            for (int32_t i = b; i < e; i += 32) {
+                v[0][lane] = cm;   // +0 past the last corner, which leaves the sums as they are
+                v[1][lane] = cf.x;
+                v[2][lane] = cf.y;
+                __syncwarp();
+                cm = 0.;
+                cf = mk(0., 0.);
+                if (i + 32 + lane < e) corner_values<kMixed>(a, __ldg(a.pcorner + i + 32 + lane), cm, cf);
+    #pragma unroll
+                for (int q = 0; q < 32; ++q) sum = __dadd_rn(sum, mine[q]);
+                __syncwarp();
+            }
+            const double wm = shfl(sum, 0), wx = shfl(sum, 1), wy = shfl(sum, 2);
+            if (lane == who) {
+                m = wm;
+                f = mk(wx, wy);
+            }
         }
     }
     if (!live) return;

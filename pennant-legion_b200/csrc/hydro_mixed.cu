@@ -810,16 +810,16 @@ PassA pass_a_kernel(bool learned, int32_t rect_nzx, bool quads) {
 // ---------------------------------------------------------------------
 // Pass B, mixed: FP32 corner inputs summed in FP64
 // ---------------------------------------------------------------------
-template <bool kRect>
+template <fp64::PointKind kKind>
 __global__ void __launch_bounds__(kPointThreads) pass_b_mixed(DevArrays a, HydroConst c) {
     pdl_wait();
     const Ctl* ctl = a.ctl;
     if (skip_cycle(ctl)) return;
     const int64_t p = (int64_t)blockIdx.x * kPointThreads + threadIdx.x;
-    if (kRect) {
+    if (kKind == fp64::kRectPoints) {
         if (p < a.nump) fp64::pass_b_point_rect<true>(a, c, ctl->cycle & 1, ctl->dt, p, a.rect_nzx, a.numz / a.rect_nzx);
     } else {
-        fp64::pass_b_point_csr<true>(a, c, ctl->cycle & 1, ctl->dt, p, p < a.nump);
+        fp64::pass_b_point_csr<true, kKind == fp64::kPointsOfMany>(a, c, ctl->cycle & 1, ctl->dt, p, p < a.nump);
     }
 }
 
@@ -872,6 +872,7 @@ __global__ void __launch_bounds__(kBatchZT, 4) batch_pass_a_mixed(BatchDev b) {
     fold.flush(b);
 }
 
+template <bool kMany>
 __global__ void __launch_bounds__(kBatchThreads) batch_point_pass_mixed(BatchDev b) {
     pdl_wait();
     for (int t = blockIdx.x; t < b.nptiles; t += gridDim.x) {
@@ -887,7 +888,7 @@ __global__ void __launch_bounds__(kBatchThreads) batch_point_pass_mixed(BatchDev
                     fp64::pass_b_point_rect<true>(b.a, c, cur, ctl.dt, p, tile.nzx, tile.nzy, tile.po,
                                                   4 * (int64_t)tile.zo);
             } else {
-                fp64::pass_b_point_csr<true>(b.a, c, cur, ctl.dt, p, p < tile.end);
+                fp64::pass_b_point_csr<true, kMany>(b.a, c, cur, ctl.dt, p, p < tile.end);
             }
         }
     }
@@ -942,8 +943,9 @@ cudaError_t launch_cycle_mixed_impl(const DevArrays& a, const HydroConst& c, cud
         if (ev) cudaEventRecord(ev[2], stream);
     }
     if (phases & kPhaseAdvance) {
-        chk(launch_pdl(a.rect_nzx > 0 ? pass_b_mixed<true> : pass_b_mixed<false>, pb, kPointThreads, 0, stream, a,
-                       c));
+        chk(launch_pdl(a.rect_nzx > 0 ? pass_b_mixed<fp64::kRectPoints>
+                                      : (a.many ? pass_b_mixed<fp64::kPointsOfMany> : pass_b_mixed<fp64::kPointsOfFew>),
+                       pb, kPointThreads, 0, stream, a, c));
         if (ev) cudaEventRecord(ev[3], stream);
         launch_pass_c(a, c, true, stream);   // its last CTA ends the cycle
         if (ev) cudaEventRecord(ev[4], stream);
@@ -974,7 +976,7 @@ cudaError_t launch_batch_pass_a_mixed(const BatchDev& b, bool all_quads, cudaStr
 }
 
 cudaError_t launch_batch_point_pass_mixed(const BatchDev& b, int grid, cudaStream_t stream) {
-    return launch_pdl(batch_point_pass_mixed, grid, kBatchThreads, 0, stream, b);
+    return launch_pdl(b.a.many ? batch_point_pass_mixed<true> : batch_point_pass_mixed<false>, grid, kBatchThreads, 0, stream, b);
 }
 
 cudaError_t prepare_learned_kernels() {
