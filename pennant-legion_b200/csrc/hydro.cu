@@ -320,7 +320,7 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
     pnt_status st = PNT_OK;
     if ((st = h->alloc(&zfirst, nz)) || (st = h->alloc(&znump, nz)) || (st = h->alloc(&mapsp1, ns)) ||
         (st = h->alloc(&smf, ns)) || (st = h->alloc(&poff, np + 1)) || (st = h->alloc(&pcorner, m.pcorner.size())) ||
-        (st = h->alloc(&mask, np + 2)) || (st = h->alloc(&zone_bc, nz)) || (st = h->alloc(&a.px[0], np)) || (st = h->alloc(&a.px[1], np)) ||
+        (st = h->alloc(&mask, np + 2)) || (st = h->alloc(&a.px[0], np)) || (st = h->alloc(&a.px[1], np)) ||
         (st = h->alloc(&a.pu[0], np)) || (st = h->alloc(&a.pu[1], np)) || (st = h->alloc(&a.zm, nz + 2)) ||
         (st = h->alloc(&a.zr, nz + 2)) || (st = h->alloc(&a.ze, nz + 2)) || (st = h->alloc(&a.zetot, nz + 2)) ||
         (st = h->alloc(&a.zwrate, nz + 2)) || (st = h->alloc(&a.zvol, nz + 2)) || (st = h->alloc(&a.zp, nz + 2)) ||
@@ -337,6 +337,7 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
     a.poff = poff;
     a.pcorner = pcorner;
     a.bcmask = mask;
+    if (pass_c_reads_words(a.rect_nzx, c.nbc, a.numz) && (st = h->alloc(&zone_bc, nz))) return st;
     a.zone_bc = zone_bc;
     if (m.is_piece) {
         // a piece: halo corner slots follow the local sides in cmass/cforce
@@ -396,7 +397,7 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
         (e = cudaMemsetAsync(a.px[1], 0, np * 16, s)) ||
         (e = cudaMemsetAsync(a.pu[1], 0, np * 16, s)))
         return fail(PNT_ERR_CUDA, "memset: %s", cudaGetErrorString(e));
-    if (a.rect_nzx > 0 && (e = launch_find_zone_bc(a, zone_bc, s)))
+    if (zone_bc && (e = launch_find_zone_bc(a, zone_bc, s)))
         return fail(PNT_ERR_CUDA, "boundary zones: %s", cudaGetErrorString(e));
     CUDA_TRY(cudaStreamSynchronize(s));
     *h->ctl_host = ctl;

@@ -99,7 +99,7 @@ struct DevArrays {
     // -dvovmax, inverted sides in A, in C] here instead of ending the cycle
     // (nullptr for a single piece)
     double* piece_red;
-    const uint16_t* zone_bc;  // [numz] the BC plane masks of the zone's points in a word (pass C on rect meshes)
+    const uint16_t* zone_bc;  // [numz] the BC plane masks of the zone's points in a word (pass C's row tiles)
     int32_t many;             // a point has more than kManyCorners corners
 };
 
@@ -184,7 +184,9 @@ cudaError_t prepare_learned_kernels();
 cudaError_t prepare_pass_c(bool mixed, bool quads, int32_t rect_nzx, int32_t nbc, int32_t numz, int nsm,
                            int32_t* grid);
 void launch_pass_c(const DevArrays& a, const HydroConst& c, bool mixed, cudaStream_t stream);
-// a.zone_bc from the mesh and the points' masks (pass_c.cu).
+// Whether pass C reads a.zone_bc, and a.zone_bc from the mesh and the points'
+// masks (pass_c.cu).
+bool pass_c_reads_words(int32_t rect_nzx, int32_t nbc, int32_t numz);
 cudaError_t launch_find_zone_bc(const DevArrays& a, uint16_t* zone_bc, cudaStream_t stream);
 // Pass A of the FP64 cycle (hydro_fp64.cu) and of the mixed or learned cycle
 // (hydro_mixed.cu): raises the kernel's shared-memory limit on the current

@@ -249,8 +249,7 @@ __global__ void __launch_bounds__(kSmallThreads) pass_c_small(DevArrays a, Hydro
     fp64::end_cycle_if_last(a, c);
 }
 
-// The BC plane masks of each zone's points in a word (not read where there are
-// more than kWordPlanes planes).
+// The BC plane masks of each zone's points in a word.
 __global__ void find_zone_bc(DevArrays a, uint16_t* zone_bc) {
     const int64_t z = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (z >= a.numz) return;
@@ -305,6 +304,10 @@ cudaError_t prepare_pass_c(bool mixed, bool quads, int32_t rect_nzx, int32_t nbc
         return cudaSuccess;
     }
     return tiles::prepare(pick_kernel(mixed, quads), stagedc::kTile, stagedc::kSmemBytes, numz, nsm, grid);
+}
+
+bool pass_c_reads_words(int32_t rect_nzx, int32_t nbc, int32_t numz) {
+    return rect_nzx > 0 && numz > kSmallZones && nbc <= kWordPlanes;
 }
 
 cudaError_t launch_find_zone_bc(const DevArrays& a, uint16_t* zone_bc, cudaStream_t stream) {
