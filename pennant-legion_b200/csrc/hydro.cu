@@ -313,7 +313,8 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
             if (e != cudaSuccess) return fail(PNT_ERR_CUDA, "pass A setup: %s", cudaGetErrorString(e));
             if (pnt_status st = h->alloc(&a.redo, (size_t)ntiles)) return st;
         } else {
-            e = prepare_pass_a_mixed(p.precision == PNT_PREC_LEARNED, a.rect_nzx, a.quads != 0, a.numz, nsm, &a.gridA);
+            e = prepare_pass_a_mixed(p.precision == PNT_PREC_LEARNED, a.rect_nzx, a.quads != 0, a.numz, nsm, &a.gridA,
+                                     &a.zone_threads);
             if (e != cudaSuccess) return fail(PNT_ERR_CUDA, "pass A setup: %s", cudaGetErrorString(e));
         }
     }

@@ -94,13 +94,14 @@ struct DevArrays {
     int32_t closure_grid;   // CTAs of the persistent closure pass
     uint32_t* redo;         // FP64 pass A: the zones of each warp tile that are formed again (hydro_fp64.cu)
     int32_t gridC;          // CTAs of the persistent pass C (pass_c_staged.cuh)
-    int32_t gridA;          // CTAs of the persistent pass A
+    int32_t gridA;          // CTAs of pass A
     // multi-piece runs: pass C's last CTA writes this piece's [dtnew,
     // -dvovmax, inverted sides in A, in C] here instead of ending the cycle
     // (nullptr for a single piece)
     double* piece_red;
     const uint16_t* zone_bc;  // [numz] the BC plane masks of the zone's points in a word (pass C's row tiles)
     int32_t many;             // a point has more than kManyCorners corners
+    int32_t zone_threads;     // mixed / learned pass A: pass_a_mixed_threads, not the warp walk
 };
 
 constexpr int kZoneThreads = 256;   // pass A: 64 zones x 4 side lanes per block
@@ -193,7 +194,8 @@ cudaError_t launch_find_zone_bc(const DevArrays& a, uint16_t* zone_bc, cudaStrea
 // device and returns its persistent grid (and the tiles a.redo holds a word
 // for).
 cudaError_t prepare_pass_a_fp64(int32_t rect_nzx, bool quads, int32_t numz, int nsm, int32_t* grid, int32_t* ntiles);
-cudaError_t prepare_pass_a_mixed(bool learned, int32_t rect_nzx, bool quads, int32_t numz, int nsm, int32_t* grid);
+cudaError_t prepare_pass_a_mixed(bool learned, int32_t rect_nzx, bool quads, int32_t numz, int nsm, int32_t* grid,
+                                 int32_t* zone_threads);
 
 // Device state of a pnt_hydro for the closure harvest (closure.cu).
 struct HydroAccess {

@@ -157,6 +157,15 @@ __device__ __forceinline__ void qcs_sfq_fp64_zone(const DevArrays& a, const Hydr
     }
 }
 
+// An edge's length and its reciprocal.  The instructions are named, since the
+// compiler took 1 / sqrt(x) as one or as two of them from one instance of the
+// zone body to the next, and the forms of pass A have to agree bit for bit.
+__device__ __forceinline__ void edge_length(float2 d, float& len, float& inv) {
+    const float x = __fmaf_rn(d.x, d.x, __fmul_rn(d.y, d.y));
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(len) : "f"(x));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(x));
+}
+
 // Per-side values parked in the thread's shared-memory slots between their
 // computation and their last use ([side][thread]: conflict-free).
 struct SideSpill {
@@ -183,6 +192,22 @@ struct RecSink {
     int* count;
     float4* base;
     int mask;
+};
+
+// A zone of a rect-numbered mesh, read as fp64::GlobalZoneIn reads others: its
+// points from its index.
+struct RectZoneIn {
+    const DevArrays& a;
+    int cur;
+    const zstage::Idx& ix;
+    __device__ __forceinline__ double2 x0(int k) const { return a.px[cur][ix.p[k]]; }
+    __device__ __forceinline__ double2 u0(int k) const { return a.pu[cur][ix.p[k]]; }
+    __device__ __forceinline__ double mf(int k) const { return __ldg(a.smf + ix.s0 + k); }
+    __device__ __forceinline__ double zm() const { return a.zm[ix.z]; }
+    __device__ __forceinline__ double zr() const { return a.zr[ix.z]; }
+    __device__ __forceinline__ double ze() const { return a.ze[ix.z]; }
+    __device__ __forceinline__ double zwrate() const { return a.zwrate[ix.z]; }
+    __device__ __forceinline__ double zvol() const { return a.zvol[ix.z]; }
 };
 
 // nbad counts the zone's inverted sides; cnt[3]: its corners without
@@ -287,8 +312,7 @@ __device__ __forceinline__ void pass_a_mixed_zone(const DevArrays& a, const Hydr
     for (int k = 0; k < N; ++k) {
         const int nk = (k + 1 == N) ? 0 : k + 1;
         ex[k] = fmul(0.5f, fadd(r[k], r[nk]));
-        elen[k] = flen(fsub(r[nk], r[k]));
-        rinv[k] = 1.f / elen[k];
+        edge_length(fsub(r[nk], r[k]), elen[k], rinv[k]);
         zdl = fminf(zdl, fac * (float)sa[k] / elen[k]);
     }
 
@@ -744,8 +768,8 @@ __device__ __forceinline__ void closure_add_counts(const DevArrays& a, const uns
         atomicAdd(a.closure_counts + kClassZones * 64 + (blockIdx.x & 63), (unsigned long long)zones);
 }
 
-// Pass A: one warp a CTA, 8 an SM, each walking tiles of 32 zones through
-// two stages of its own (zone_stage.cuh).  1920^2 Sedov, mixed / learned:
+// Pass A, the warp walk: one warp a CTA, 8 an SM, each walking tiles of 32 zones
+// through two stages of its own (zone_stage.cuh).  1920^2 Sedov, mixed / learned:
 // 0.251 / 0.218 ms, against 0.291 / 0.258 ms for CTAs of 96 zones with a
 // barrier a tile (12 warps an SM, 168 registers); with 12 or 16 warps this way
 // 0.34-0.40 ms (spills, and stages that leave 30 KB of L1).  The EOS's two
@@ -797,6 +821,69 @@ __global__ void __launch_bounds__(32, 8) pass_a_mixed(DevArrays a, HydroConst c)
     fp64::warp_to_cycle<true>(a.cyc_red, zdthyd, bad);
 }
 
+// Pass A, one thread a zone with plain loads, a CTA per 128 zones, 16 warps an
+// SM (128 registers, 64-80 B of spills): its CTAs go to the SMs as these come
+// free, and two rounds of the warp walk above are one of its own.  Cycles,
+// this one / the warp walk: rect 225^2 Noh 20.0 / 21.4 us, Sedov 22.2 / 23.1
+// (21.4 and 24.5 with the CTAs of 96 zones).  Without the rect numbering the
+// walk reads indices before its copies and gains nothing on long runs of tiles
+// either; pass A, this one / the walk: quads 300^2 Sedov 18.3 / 23.4 us, 480^2
+// 26.2 / 30.1, 1024^2 88 / 98 (Noh 80.6 / 76.3), 300 x 400 pie 18.2 / 22.7, 800 x
+// 1000 pie 70.7 / 79.8.  In one round the walk is ahead (cycle of 150^2 quads,
+// Noh 18.0 / 17.5, Sedov 19.6 / 19.0 us), and on rect meshes of more rounds, and
+// in the learned cycle, the two change places with the flow (600^2 mixed, Sedov
+// 58.9 / 69.5, Noh 54.6 / 56.3; 2880 x 288 Leblanc 105.8 / 99.7; 225^2 learned
+// 33.2 / 33.0, Noh 47.2 / 47.8).
+constexpr int kThreadsA = 128;
+template <zstage::MeshKind kKind, bool kLearned>
+__global__ void __launch_bounds__(kThreadsA, 4) pass_a_mixed_threads(DevArrays a, HydroConst c) {
+    pdl_wait();
+    const Ctl* ctl = a.ctl;
+    if (skip_cycle(ctl)) return;
+    const int32_t z = (int32_t)(blockIdx.x * kThreadsA + threadIdx.x);
+    double zdthyd = 1.e99;
+    int bad = 0;
+    int cnt[3] = {0, 0, 0};
+    __shared__ double2 s_sfp[4 * kThreadsA];
+    __shared__ float2 s_sft[4 * kThreadsA];
+    const SideSpill sp{s_sfp, s_sft, (int)threadIdx.x, kThreadsA};
+    if (z < a.numz) {
+        const int cur = ctl->cycle & 1;
+        const double dt = ctl->dt;
+        const RecSink sink{a.closure_nrec, reinterpret_cast<float4*>(a.closure_rec), 0x7fffffff};
+        if (kKind == zstage::kRect) {
+            const zstage::Idx ix = zstage::rect_idx(z, a.rect_nzx, 0, 0);
+            const RectZoneIn in{a, cur, ix};
+            pass_a_mixed_zone<4, kLearned>(a, c, in, cur, dt, z, ix.s0, zdthyd, bad, cnt, sp, sink);
+        } else if (kKind == zstage::kQuads) {
+            const fp64::GlobalZoneIn in{a, cur, z, 4 * z};
+            pass_a_mixed_zone<4, kLearned>(a, c, in, cur, dt, z, 4 * z, zdthyd, bad, cnt, sp, sink);
+        } else {
+            const int n = a.znump[z];
+            const int64_t s0 = a.zfirst[z];
+            const fp64::GlobalZoneIn in{a, cur, z, s0};
+            if (n == 4) pass_a_mixed_zone<4, kLearned>(a, c, in, cur, dt, z, s0, zdthyd, bad, cnt, sp, sink);
+            else pass_a_mixed_zone<3, kLearned>(a, c, in, cur, dt, z, s0, zdthyd, bad, cnt, sp, sink);
+        }
+    }
+    if constexpr (kLearned) {
+        constexpr int kCounted[3] = {kClassZero, kClassDead, kClassAcute};
+        __shared__ unsigned count[3];
+        if (threadIdx.x < 3) count[threadIdx.x] = 0;
+        __syncthreads();
+        for (int q = 0; q < 3; ++q) {
+            const unsigned t = __reduce_add_sync(kFull, (unsigned)cnt[q]);
+            if ((threadIdx.x & 31) == 0 && t) atomicAdd(count + q, t);
+        }
+        __syncthreads();
+        if (threadIdx.x < 3 && count[threadIdx.x])
+            atomicAdd(a.closure_counts + kCounted[threadIdx.x] * 64 + (blockIdx.x & 63),
+                      (unsigned long long)count[threadIdx.x]);
+    }
+    const int nbad = tiles::block_isum<kThreadsA>(bad);
+    fp64::block_to_cycle<true, kThreadsA>(a.cyc_red, zdthyd, nbad);
+}
+
 using PassA = void (*)(DevArrays, HydroConst);
 template <bool kLearned>
 PassA pass_a_kernel(int32_t rect_nzx, bool quads) {
@@ -805,6 +892,11 @@ PassA pass_a_kernel(int32_t rect_nzx, bool quads) {
 }
 PassA pass_a_kernel(bool learned, int32_t rect_nzx, bool quads) {
     return learned ? pass_a_kernel<true>(rect_nzx, quads) : pass_a_kernel<false>(rect_nzx, quads);
+}
+PassA pass_a_threads_kernel(bool learned, int32_t rect_nzx, bool quads) {
+    if (rect_nzx > 0) return pass_a_mixed_threads<zstage::kRect, false>;   // mixed meshes alone (prepare_pass_a_mixed)
+    if (learned) return quads ? pass_a_mixed_threads<zstage::kQuads, true> : pass_a_mixed_threads<zstage::kGeneral, true>;
+    return quads ? pass_a_mixed_threads<zstage::kQuads, false> : pass_a_mixed_threads<zstage::kGeneral, false>;
 }
 
 // ---------------------------------------------------------------------
@@ -937,7 +1029,11 @@ cudaError_t launch_cycle_mixed_impl(const DevArrays& a, const HydroConst& c, cud
     };
     if (phases & kPhaseForces) {
         if (ev) cudaEventRecord(ev[0], stream);
-        chk(launch_pdl(pass_a_kernel(learned, a.rect_nzx, a.quads != 0), a.gridA, 32, zstage::kSmem, stream, a, c));
+        if (a.zone_threads)
+            chk(launch_pdl(pass_a_threads_kernel(learned, a.rect_nzx, a.quads != 0), a.gridA, kThreadsA, 0, stream, a,
+                           c));
+        else
+            chk(launch_pdl(pass_a_kernel(learned, a.rect_nzx, a.quads != 0), a.gridA, 32, zstage::kSmem, stream, a, c));
         if (ev) cudaEventRecord(ev[1], stream);
         if (learned) chk(launch_pdl(closure_pass, a.closure_grid, kCpThreads, kCpSmemBytes, stream, a, c));
         if (ev) cudaEventRecord(ev[2], stream);
@@ -966,8 +1062,15 @@ cudaError_t launch_cycle_learned(const DevArrays& a, const HydroConst& c, cudaSt
     return launch_cycle_mixed_impl(a, c, stream, ev, true, phases);
 }
 
-cudaError_t prepare_pass_a_mixed(bool learned, int32_t rect_nzx, bool quads, int32_t numz, int nsm, int32_t* grid) {
-    return zstage::prepare(pass_a_kernel(learned, rect_nzx, quads), rect_nzx, numz, nsm, grid);
+cudaError_t prepare_pass_a_mixed(bool learned, int32_t rect_nzx, bool quads, int32_t numz, int nsm, int32_t* grid,
+                                 int32_t* zone_threads) {
+    const cudaError_t e = zstage::prepare(pass_a_kernel(learned, rect_nzx, quads), rect_nzx, numz, nsm, grid);
+    const int32_t tiles = (numz + zstage::kT - 1) / zstage::kT;
+    const int32_t round = 8 * nsm;   // the warp walk's warps at a time
+    // the limits: pass_a_mixed_threads
+    *zone_threads = tiles > round && (rect_nzx <= 0 || (!learned && tiles <= 2 * round));
+    if (*zone_threads) *grid = (numz + kThreadsA - 1) / kThreadsA;
+    return e;
 }
 
 cudaError_t launch_batch_pass_a_mixed(const BatchDev& b, bool all_quads, cudaStream_t stream) {
