@@ -214,7 +214,10 @@ struct RectZoneIn {
 // compression, in the dead zone, in an acute zone (learned cycle).
 // in: the zone's inputs (fp64::GlobalZoneIn, or a row tile's shared-memory
 // stage); sink: where a zone with deferred corners is recorded (learned).
-template <int N, bool kLearned, typename In, typename Park>
+// kStraight: the EOS's quotients in straight-line code, which gains where the
+// kernel has the registers for it and costs 1-2% at 128 (800 x 1000 pie 71.3
+// against 69.9 us, batches 0.5-1%); the bits are the same.
+template <int N, bool kLearned, bool kStraight, typename In, typename Park>
 __device__ __forceinline__ void pass_a_mixed_zone(const DevArrays& a, const HydroConst& c, const In& in, int cur,
                                                   double dt, int64_t z, int64_t s0, double& zdthyd, int& nbad,
                                                   int* cnt, const Park& sp, const RecSink& sink = RecSink{}) {
@@ -266,20 +269,23 @@ __device__ __forceinline__ void pass_a_mixed_zone(const DevArrays& a, const Hydr
     const double q = c.gm1 * pre;
     const double csqd = dmax(c.ssmin2, pre + q);
     const double bulk = zr * csqd;
-    ieee::Guard g;
     auto eos_num = [&](double minv, double dv) {
         const double src = zwrate * dth * minv;
         return per * src - zr * bulk * dv;
     };
-    double minv = ieee::rcp(zm, g);
-    double dv = (zvolp - zvol0) * minv;
-    double denom = 1. + 0.5 * per * dv;
-    double dp = ieee::quot1(eos_num(minv, dv), denom, g);
-    if (!g.ok()) {   // out of the straight-line form's range (ieee_div.cuh): the operators
-        minv = 1. / zm;
-        dv = (zvolp - zvol0) * minv;
-        denom = 1. + 0.5 * per * dv;
-        dp = eos_num(minv, dv) / denom;
+    double dp = 0.;
+    bool formed = false;
+    if constexpr (kStraight) {
+        ieee::Guard g;
+        const double minv = ieee::rcp(zm, g);
+        const double dv = (zvolp - zvol0) * minv;
+        dp = ieee::quot1(eos_num(minv, dv), 1. + 0.5 * per * dv, g);
+        formed = g.ok();
+    }
+    if (!formed) {   // or out of the straight-line form's range (ieee_div.cuh): the operators
+        const double minv = 1. / zm;
+        const double dv = (zvolp - zvol0) * minv;
+        dp = eos_num(minv, dv) / (1. + 0.5 * per * dv);
     }
     const double zp = __fma_rn(c.gm1 * zr, e, dp);
     const float zssf = sqrtf((float)csqd);
@@ -802,9 +808,9 @@ __global__ void __launch_bounds__(32, 8) pass_a_mixed(DevArrays a, HydroConst c)
         double v = 1.e99;
         int zc[3] = {0, 0, 0};   // the zone's own corner classes (an acute zone overwrites them)
         if (kKind != zstage::kGeneral || n == 4)
-            pass_a_mixed_zone<4, kLearned>(a, c, in, cur, dt, z, s0, v, bad, zc, sp, sink);
+            pass_a_mixed_zone<4, kLearned, true>(a, c, in, cur, dt, z, s0, v, bad, zc, sp, sink);
         else
-            pass_a_mixed_zone<3, kLearned>(a, c, in, cur, dt, z, s0, v, bad, zc, sp, sink);
+            pass_a_mixed_zone<3, kLearned, true>(a, c, in, cur, dt, z, s0, v, bad, zc, sp, sink);
         zdthyd = dmin(zdthyd, v);
 #pragma unroll
         for (int q = 0; q < 3; ++q) cnt[q] += zc[q];
@@ -854,33 +860,34 @@ __global__ void __launch_bounds__(kThreadsA, 4) pass_a_mixed_threads(DevArrays a
         if (kKind == zstage::kRect) {
             const zstage::Idx ix = zstage::rect_idx(z, a.rect_nzx, 0, 0);
             const RectZoneIn in{a, cur, ix};
-            pass_a_mixed_zone<4, kLearned>(a, c, in, cur, dt, z, ix.s0, zdthyd, bad, cnt, sp, sink);
+            pass_a_mixed_zone<4, kLearned, false>(a, c, in, cur, dt, z, ix.s0, zdthyd, bad, cnt, sp, sink);
         } else if (kKind == zstage::kQuads) {
             const fp64::GlobalZoneIn in{a, cur, z, 4 * z};
-            pass_a_mixed_zone<4, kLearned>(a, c, in, cur, dt, z, 4 * z, zdthyd, bad, cnt, sp, sink);
+            pass_a_mixed_zone<4, kLearned, false>(a, c, in, cur, dt, z, 4 * z, zdthyd, bad, cnt, sp, sink);
         } else {
             const int n = a.znump[z];
             const int64_t s0 = a.zfirst[z];
             const fp64::GlobalZoneIn in{a, cur, z, s0};
-            if (n == 4) pass_a_mixed_zone<4, kLearned>(a, c, in, cur, dt, z, s0, zdthyd, bad, cnt, sp, sink);
-            else pass_a_mixed_zone<3, kLearned>(a, c, in, cur, dt, z, s0, zdthyd, bad, cnt, sp, sink);
+            if (n == 4) pass_a_mixed_zone<4, kLearned, false>(a, c, in, cur, dt, z, s0, zdthyd, bad, cnt, sp, sink);
+            else pass_a_mixed_zone<3, kLearned, false>(a, c, in, cur, dt, z, s0, zdthyd, bad, cnt, sp, sink);
         }
     }
+    __shared__ unsigned wcount[kLearned ? kThreadsA / 32 : 1][3];
     if constexpr (kLearned) {
-        constexpr int kCounted[3] = {kClassZero, kClassDead, kClassAcute};
-        __shared__ unsigned count[3];
-        if (threadIdx.x < 3) count[threadIdx.x] = 0;
-        __syncthreads();
         for (int q = 0; q < 3; ++q) {
             const unsigned t = __reduce_add_sync(kFull, (unsigned)cnt[q]);
-            if ((threadIdx.x & 31) == 0 && t) atomicAdd(count + q, t);
+            if ((threadIdx.x & 31) == 0) wcount[threadIdx.x >> 5][q] = t;
         }
-        __syncthreads();
-        if (threadIdx.x < 3 && count[threadIdx.x])
-            atomicAdd(a.closure_counts + kCounted[threadIdx.x] * 64 + (blockIdx.x & 63),
-                      (unsigned long long)count[threadIdx.x]);
     }
-    const int nbad = tiles::block_isum<kThreadsA>(bad);
+    const int nbad = tiles::block_isum<kThreadsA>(bad);   // its barrier also orders wcount
+    if constexpr (kLearned) {
+        constexpr int kCounted[3] = {kClassZero, kClassDead, kClassAcute};
+        if (threadIdx.x < 3) {
+            unsigned t = 0;
+            for (int w = 0; w < kThreadsA / 32; ++w) t += wcount[w][threadIdx.x];
+            if (t) atomicAdd(a.closure_counts + kCounted[threadIdx.x] * 64 + (blockIdx.x & 63), (unsigned long long)t);
+        }
+    }
     fp64::block_to_cycle<true, kThreadsA>(a.cyc_red, zdthyd, nbad);
 }
 
@@ -950,13 +957,13 @@ __global__ void __launch_bounds__(kBatchZT, 4) batch_pass_a_mixed(BatchDev b) {
         int cnt[3] = {0, 0, 0};
         if (kAllQuads || tile.quads) {
             const fp64::GlobalZoneIn in{b.a, cur, z, 4 * z};
-            pass_a_mixed_zone<4, false>(b.a, c, in, cur, dt, z, 4 * z, v, fold.bad, cnt, sp);
+            pass_a_mixed_zone<4, false, false>(b.a, c, in, cur, dt, z, 4 * z, v, fold.bad, cnt, sp);
         } else {
             const int n = b.a.znump[z];
             const int64_t s0 = b.a.zfirst[z];
             const fp64::GlobalZoneIn in{b.a, cur, z, s0};
-            if (n == 4) pass_a_mixed_zone<4, false>(b.a, c, in, cur, dt, z, s0, v, fold.bad, cnt, sp);
-            else pass_a_mixed_zone<3, false>(b.a, c, in, cur, dt, z, s0, v, fold.bad, cnt, sp);
+            if (n == 4) pass_a_mixed_zone<4, false, false>(b.a, c, in, cur, dt, z, s0, v, fold.bad, cnt, sp);
+            else pass_a_mixed_zone<3, false, false>(b.a, c, in, cur, dt, z, s0, v, fold.bad, cnt, sp);
         }
         fold.v = dmin(fold.v, v);
     }
