@@ -354,7 +354,8 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
             (st = h->alloc(&a.piece_red, 4)))
             return st;
         if (h->nsend > 0)
-            CUDA_TRY(cudaMemcpy(h->send_side, m.send_side.data(), (size_t)h->nsend * 4, cudaMemcpyHostToDevice));
+            CUDA_TRY(cudaMemcpyAsync(h->send_side, m.send_side.data(), (size_t)h->nsend * 4, cudaMemcpyHostToDevice,
+                                     h->stream));
     }
 
     // Driver::run start: time 0, cycle 0 and calcGlobalDt for cycle 0
@@ -839,7 +840,7 @@ pnt_status pnt_hydro_set_closure(pnt_hydro* h, const pnt_closure* c, int32_t mod
         if (pnt_status st = h->alloc(&img, kImgBytes)) return st;
         if (pnt_status st = h->alloc(&rec, (size_t)h->numz * kZoneRecF4 * 4)) return st;
         if (pnt_status st = h->alloc(&nrec, 1)) return st;
-        CUDA_TRY(cudaMemset(nrec, 0, sizeof(int32_t)));
+        CUDA_TRY(cudaMemsetAsync(nrec, 0, sizeof(int32_t), h->stream));
         CUDA_TRY(prepare_learned_kernels());
         int nsm = 148;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
