@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kSmallThreads) pass_a_small(DevArrays a, Hydro
     }
     __syncwarp();
     const int nbad = tiles::block_isum<kSmallThreads>(bad);
-    block_to_cycle<true, kSmallThreads>(a.cyc_red, zdthyd, nbad);
+    block_to_cycle<true, kSmallThreads>(a.cyc_red, dmin(1.e99, zdthyd), nbad);   // a NaN is left out
 }
 
 template <PointKind kKind>

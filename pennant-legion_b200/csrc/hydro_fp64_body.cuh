@@ -127,8 +127,8 @@ __device__ __forceinline__ double dkey_value(long long k) {
 
 // A block's share of the cycle reductions (one mesh): its minimum zone dt
 // (pass A) or maximum |dV/V0| (pass C) into cyc_red[0] / [1], its inverted
-// sides into [2] / [3].  A NaN result is left out, as the serial fold leaves
-// NaN out after its first value.
+// sides into [2] / [3].  No v is a NaN: the serial fold leaves NaN out after
+// its first value, 1e99 or 1e-99, and the callers do.
 template <bool kPassA, int kThreads>
 __device__ __forceinline__ void block_to_cycle(long long* cyc_red, double v, int nbad) {
     const double r = block_fold_value<kPassA, kThreads>(v);

@@ -888,7 +888,7 @@ __global__ void __launch_bounds__(kThreadsA, 4) pass_a_mixed_threads(DevArrays a
             if (t) atomicAdd(a.closure_counts + kCounted[threadIdx.x] * 64 + (blockIdx.x & 63), (unsigned long long)t);
         }
     }
-    fp64::block_to_cycle<true, kThreadsA>(a.cyc_red, zdthyd, nbad);
+    fp64::block_to_cycle<true, kThreadsA>(a.cyc_red, dmin(1.e99, zdthyd), nbad);   // a NaN is left out
 }
 
 using PassA = void (*)(DevArrays, HydroConst);

@@ -58,6 +58,17 @@ def test_one_zone_s_energy(mesh, value):
         assert s["dtnew"] == 0.0
 
 
+@pytest.mark.parametrize("mesh", MESHES, ids=lambda m: f"{m[0]}-{m[1]}-{m[2]}")
+def test_a_zone_whose_dt_is_no_number(mesh):
+    # without linear viscosity an infinite sound speed gives 0 x inf; the
+    # smallest dt of the mesh is left to zones next to that one
+    def change(o):
+        z = np.arange(o.numz)
+        return {"ze": np.where(z == 32, np.inf, np.where(z // 32 == 1, 50.0, 0.01))}
+    s = check_one_cycle(deck_text(mesh, dtinit=1e-9).replace("q1 0.1", "q1 0.0"), change)
+    assert 0.0 < s["dtnew"] < 1e90
+
+
 def test_energy_whose_square_term_overflows():
     # (gamma - 1)^2 rho^2 e overflows for finite e and pressure
     text = deck_text(("rect", 33, 20), dtinit=1e-200) + "rinit 1.0e3\n"
