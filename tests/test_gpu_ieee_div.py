@@ -4,7 +4,9 @@ bit for bit, wherever their guard accepts the operands; numpy's are the oracle.
 Operands: random ones over and beyond the guarded ranges, with random, sparse
 and nearly full mantissas, and for roots every x whose root lies within 2^-45
 ulp of the midpoint of two doubles (there an error below an ulp's 2^-53, which
-the method allows before its last rounding, could show)."""
+the method allows before its last rounding, could show); for quotients, ones
+whose distance from such a midpoint is a few times the least that there is; and
+the approximations that both start from, at every mantissa they distinguish."""
 import ctypes
 import math
 import os
@@ -39,6 +41,13 @@ __global__ void roots(const double* x, long n, double* r, int* ok) {
     r[i] = ieee::root(x[i], g);
     ok[i] = g.ok() ? 1 : 0;
 }
+__global__ void starts(const double* x, long n, double* y, double* z, int* ok) {
+    const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y[i]) : "d"(x[i]));
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(z[i]) : "d"(x[i]));
+    ok[i] = 1;
+}
 template <typename F>
 static int run(int nin, const double* const* in, int nout, double* const* out, int* ok, long n, F launch) {
     double* d[8] = {};
@@ -59,6 +68,11 @@ extern "C" int run_quots(const double* a, const double* b, long n, double* q, do
     const double* in[2] = {a, b};
     double* out[3] = {q, q0, inv};
     return run(2, in, 3, out, ok, n, [&](double** d, int* o) { quots<<<(n + 255) / 256, 256>>>(d[0], d[1], n, d[2], d[3], d[4], o); });
+}
+extern "C" int run_starts(const double* x, long n, double* y, double* z, int* ok) {
+    const double* in[1] = {x};
+    double* out[2] = {y, z};
+    return run(1, in, 2, out, ok, n, [&](double** d, int* o) { starts<<<(n + 255) / 256, 256>>>(d[0], n, d[1], d[2], o); });
 }
 extern "C" int run_roots(const double* x, long n, double* r, int* ok) {
     const double* in[1] = {x};
@@ -132,6 +146,65 @@ def test_quotients_are_the_operators(lib, kind):
         assert (ok == 7).all()
     zero = (a == 0) & ((ok & 4) != 0)
     assert ((ok[zero] & 2) != 0).all() and ((ok[zero] & 1) == 0).all()
+
+
+def _quotient_hard_cases(n, most):
+    """a, b with a / b = N / 2^53 (1 + c / (b N)), N odd of 54 bits and |c| <= most odd: c / b ulp halves
+    from the midpoint N / 2 of two doubles, where 1 / b is the nearest that a quotient can come."""
+    rng = np.random.default_rng(13)
+    a, b = [], []
+    while len(a) < n:
+        d = int(rng.integers(1 << 51, 1 << 52)) * 2 + 1   # an odd divisor of 53 bits
+        c = int(rng.integers(0, most + 1)) // 2 * 2 + 1
+        c = c if rng.integers(0, 2) else -c
+        N = (-c * pow(d, -1, 1 << 54)) % (1 << 54)
+        if N >= 1 << 53:
+            a.append((d * N + c) >> 54)
+            b.append(d)
+    return a, b
+
+
+def test_quotient_hard_cases_are_found():
+    for a, b in zip(*_quotient_hard_cases(200, 63)):
+        assert a < 1 << 53 and b < 1 << 53
+        r = (a << 54) % b   # of 2 (a / b) in units of the quotient's half ulp
+        assert min(r, b - r) <= 63 and round((a << 54) / b) >= 1 << 53
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("most", [1, 63, 4095])
+def test_quotients_next_to_midpoints(lib, most):
+    ia, ib = _quotient_hard_cases(100000, most)
+    a, b = np.array(ia, dtype=np.float64), np.array(ib, dtype=np.float64)
+    rng = np.random.default_rng(14)
+    s = rng.integers(-150, 150, a.size)   # anywhere in the divisors' range
+    a = np.ldexp(a * rng.choice([-1.0, 1.0], a.size), rng.integers(-600, 200, a.size))
+    b = np.ldexp(b, s - 52)
+    n = a.size
+    q, q0, inv = (np.empty(n) for _ in range(3))
+    ok = np.empty(n, np.int32)
+    assert lib.run_quots(_ptr(a), _ptr(b), ctypes.c_long(n), _ptr(q), _ptr(q0), _ptr(inv), _ptr(ok)) == 0
+    assert (ok == 7).all()
+    assert _same(q, a / b).all() and _same(q0, a / b).all() and _same(inv, 1.0 / b).all()
+
+
+@pytest.mark.gpu
+def test_the_approximations_at_every_mantissa(lib):
+    """Both read a double's high word; |1 - b y| < 2^-19.9 and |1 - x z^2| < 2^-19.0 hold over all low words if
+    they hold at the ends, as y and z are the same for all and the products are monotonic."""
+    hi = np.arange(1 << 21, dtype=np.uint64) + np.uint64(1023 << 20)   # [1, 4): both parities of the exponent
+    lo = [hi << np.uint64(32), (hi << np.uint64(32)) | np.uint64(0xffffffff)]
+    lo.append((hi << np.uint64(32)) | np.random.default_rng(15).integers(0, 1 << 32, hi.size, dtype=np.uint64))
+    got = []
+    for bits in lo:
+        x = bits.view(np.float64)
+        y, z, ok = np.empty(x.size), np.empty(x.size), np.empty(x.size, np.int32)
+        assert lib.run_starts(_ptr(x), ctypes.c_long(x.size), _ptr(y), _ptr(z), _ptr(ok)) == 0
+        got.append((x.astype(np.longdouble), y.astype(np.longdouble), z.astype(np.longdouble)))
+    for x, y, z in got:   # 21 significant bits in y and z: the products are exact to 2^-63
+        assert (y == got[0][1]).all() and (z == got[0][2]).all()
+        assert np.abs(1 - x * y).max() < 2.0 ** -19.9
+        assert np.abs(1 - x * z * z).max() < 2.0 ** -19.0
 
 
 def _root_hard_cases(most):
