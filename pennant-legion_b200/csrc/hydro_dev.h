@@ -104,7 +104,7 @@ struct DevArrays {
     int32_t zone_threads;     // mixed / learned pass A: pass_a_mixed_threads, not the warp walk
 };
 
-constexpr int kZoneThreads = 256;   // pass A: 64 zones x 4 side lanes per block
+constexpr int kZoneThreads = 256;   // closure harvest: 64 zones x 4 side lanes per block
 constexpr int kPointThreads = 256;
 constexpr int kManyCorners = 8;     // pass B: points of more are gathered by their warp
 

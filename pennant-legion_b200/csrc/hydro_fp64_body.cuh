@@ -37,10 +37,6 @@ __device__ __forceinline__ double cross(double2 a, double2 b) { return a.x * b.y
 __device__ __forceinline__ double length(double2 v) { return sqrt(v.x * v.x + v.y * v.y); }
 __device__ __forceinline__ double length2(double2 v) { return v.x * v.x + v.y * v.y; }
 __device__ __forceinline__ double2 rotateCCW(double2 v) { return mk(-v.y, v.x); }
-__device__ __forceinline__ double2 project(double2 v, double ux, double uy) {
-    const double d = v.x * ux + v.y * uy;
-    return mk(v.x - ux * d, v.y - uy * d);
-}
 // std::min / std::max: min(a,b) = (b < a) ? b : a, max(a,b) = (a < b) ? b : a
 __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; }
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
@@ -240,7 +236,7 @@ __device__ __forceinline__ void qcs_corner(const HydroConst& c, double2 up0, dou
 // ---------------------------------------------------------------------
 // Pass A's inputs of one zone gathered from global memory: the position
 // and velocity of each side's first point (current buffer), the side mass
-// fractions and the zone fields.  The row-tile kernels read the same
+// fractions and the zone fields.  The kernels of zone_stage.cuh read the same
 // values from shared memory through an accessor of the same shape.
 struct GlobalZoneIn {
     const DevArrays& a;
@@ -739,8 +735,8 @@ __device__ __forceinline__ bool pass_a_zone_lanes(const DevArrays& a, const Hydr
 // (Hydro.cc:1235-1254, pa = f * (1 / max(m, 1e-99))) and advPosFull
 // (:1281-1306).  Written with explicit round-to-nearest operations, so the
 // result does not depend on the including file's contraction flags: the
-// FP64 and mixed cycles, the batch and the fused row-tile pass all advance
-// a point bit-identically from the same sums.
+// FP64 and mixed cycles and the batch all advance a point bit-identically
+// from the same sums.
 __device__ __forceinline__ double2 project_rn(double2 v, double ux, double uy) {
     const double d = __dadd_rn(__dmul_rn(v.x, ux), __dmul_rn(v.y, uy));
     return mk(__dsub_rn(v.x, __dmul_rn(ux, d)), __dsub_rn(v.y, __dmul_rn(uy, d)));

@@ -47,10 +47,6 @@ __device__ __forceinline__ double2 sub(double2 a, double2 b) { return mk(a.x - b
 __device__ __forceinline__ double2 smul(double r, double2 v) { return mk(v.x * r, v.y * r); }
 __device__ __forceinline__ double dot(double2 a, double2 b) { return a.x * b.x + a.y * b.y; }
 __device__ __forceinline__ double cross(double2 a, double2 b) { return a.x * b.y - a.y * b.x; }
-__device__ __forceinline__ double2 project(double2 v, double ux, double uy) {
-    const double d = v.x * ux + v.y * uy;
-    return mk(v.x - ux * d, v.y - uy * d);
-}
 __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; }
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
 
@@ -68,15 +64,6 @@ __device__ __forceinline__ float2 shflf2(float2 v, int src) {
     return fk(__shfl_sync(kFull, v.x, src), __shfl_sync(kFull, v.y, src));
 }
 
-template <typename T>
-__device__ __forceinline__ T zsum4(T v, int g, int n) {
-    T s = __shfl_sync(kFull, v, g);
-    s += __shfl_sync(kFull, v, g + 1);
-    s += __shfl_sync(kFull, v, g + 2);
-    const T d = __shfl_sync(kFull, v, g + 3);
-    if (n == 4) s += d;
-    return s;
-}
 
 __device__ __forceinline__ bool skip_cycle(const Ctl* ctl) {
     return ctl->done || ctl->cycle >= ctl->stop_at;
@@ -186,12 +173,10 @@ struct SideRegs {
 };
 
 // Where the learned cycle's pass A records a zone for the closure: record
-// i at base + (i & mask) * kZoneRecF4, i from an atomic counter (global or
-// shared memory).
+// i at base + i kZoneRecF4, i from an atomic counter.
 struct RecSink {
     int* count;
     float4* base;
-    int mask;
 };
 
 // A zone of a rect-numbered mesh, read as fp64::GlobalZoneIn reads others: its
@@ -212,8 +197,8 @@ struct RectZoneIn {
 
 // nbad counts the zone's inverted sides; cnt[3]: its corners without
 // compression, in the dead zone, in an acute zone (learned cycle).
-// in: the zone's inputs (fp64::GlobalZoneIn, or a row tile's shared-memory
-// stage); sink: where a zone with deferred corners is recorded (learned).
+// in: the zone's inputs (fp64::GlobalZoneIn, RectZoneIn, or a warp's stage,
+// zstage::ZoneIn); sink: where a zone with deferred corners is recorded (learned).
 // kStraight: the EOS's quotients in straight-line code, which gains where the
 // kernel has the registers for it and costs 1-2% at 128 (800 x 1000 pie 71.3
 // against 69.9 us, batches 0.5-1%); the bits are the same.
@@ -423,7 +408,7 @@ __device__ __forceinline__ void pass_a_mixed_zone(const DevArrays& a, const Hydr
             if (lane == leader) base = atomicAdd(sink.count, __popc(m));
             base = __shfl_sync(m, base, leader);
             const int idx = base + __popc(m & ((1u << lane) - 1u));
-            float4* rec = sink.base + (int64_t)(idx & sink.mask) * kZoneRecF4;
+            float4* rec = sink.base + (int64_t)idx * kZoneRecF4;
             const float2 r3 = (N == 4) ? r[N - 1] : fk(0.f, 0.f), u3 = (N == 4) ? uf[N - 1] : fk(0.f, 0.f);
             rec[0] = make_float4(r[0].x, r[0].y, r[1].x, r[1].y);
             rec[1] = make_float4(r[2].x, r[2].y, r3.x, r3.y);
@@ -798,7 +783,7 @@ __global__ void __launch_bounds__(32, 8) pass_a_mixed(DevArrays a, HydroConst c)
         __shared__ float2 s_sft[4 * 32];
         sp = SideSpill{s_sfp, s_sft, lane, 32};
     }
-    const RecSink sink{a.closure_nrec, reinterpret_cast<float4*>(a.closure_rec), 0x7fffffff};
+    const RecSink sink{a.closure_nrec, reinterpret_cast<float4*>(a.closure_rec)};
     double zdthyd = 1.e99;
     int bad = 0;
     int cnt[3] = {0, 0, 0};
@@ -856,7 +841,7 @@ __global__ void __launch_bounds__(kThreadsA, 4) pass_a_mixed_threads(DevArrays a
     if (z < a.numz) {
         const int cur = ctl->cycle & 1;
         const double dt = ctl->dt;
-        const RecSink sink{a.closure_nrec, reinterpret_cast<float4*>(a.closure_rec), 0x7fffffff};
+        const RecSink sink{a.closure_nrec, reinterpret_cast<float4*>(a.closure_rec)};
         if (kKind == zstage::kRect) {
             const zstage::Idx ix = zstage::rect_idx(z, a.rect_nzx, 0, 0);
             const RectZoneIn in{a, cur, ix};

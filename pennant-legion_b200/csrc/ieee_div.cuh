@@ -13,8 +13,8 @@
 //
 // Quotients (P. Markstein, IBM J. Res. Dev. 34 (1990) 111; M. Cornea, J.
 // Harrison, P. Tang, "Scientific Computing on Itanium-based Systems", 2002).
-// rcp: y0 from the reciprocal instruction, |e| = |1 - b y0| < 2^-19.9 (every
-// mantissa it can distinguish was tried), y1 = y0 (1 + e + e^2), within 0.52
+// rcp: y0 from the reciprocal instruction, |e| = |1 - b y0| < 2^-19.9 (at
+// every mantissa that it distinguishes: tests/test_gpu_ieee_div.py), y1 = y0 (1 + e + e^2), within 0.52
 // ulp of 1/b, and y = y1 + y1 (1 - b y1), which is 1/b correctly rounded by
 // Markstein's theorem unless b's mantissa is all ones; there 1/b rounds to a
 // power of two plus one ulp.  quot: q0 = a y, r = a - b q0, q = q0 + r y, the

@@ -1,7 +1,8 @@
-// zone_stage.cuh -- the FP64 pass A's inputs, a warp's 32 zones at a time,
-// through shared-memory stages that the warp fills for itself.
+// zone_stage.cuh -- pass A's inputs (the FP64 cycle's, and the mixed and
+// learned cycles'), a warp's 32 zones at a time, through shared-memory stages
+// that the warp fills for itself.
 //
-// The zone body (pass_a_zone_fast) needs about 250 registers to interleave
+// The FP64 zone body (pass_a_zone_fast) needs about 250 registers to interleave
 // its quotients without spilling, so 8 warps fit an SM, and warps that load
 // and then compute leave it idle while they load (1024^2 Sedov, 12 warps and
 // plain loads: 2.7 of 7 stalled cycles an instruction on the loads).  Here a

@@ -15,10 +15,7 @@
 // shared-memory accesses), so `cp.async.wait_group` alone orders them; no
 // block barrier inside the loop.
 //
-// Pass A gains nothing from it: one thread per zone there is bound by its
-// arithmetic (1024^2 Sedov: staged 91-105 us mixed, 195-216 us FP64, against
-// 89 and 173 us loading straight into registers, 128 and 168 registers),
-// so pass A keeps plain loads.
+// Pass A's stages are a warp's own (zone_stage.cuh).
 #pragma once
 
 #include "hydro_dev.h"
