@@ -956,7 +956,6 @@ __global__ void __launch_bounds__(kBatchZT, 4) batch_pass_a_mixed(BatchDev b) {
     fold.flush(b);
 }
 
-template <bool kMany>
 __global__ void __launch_bounds__(kBatchThreads) batch_point_pass_mixed(BatchDev b) {
     pdl_wait();
     for (int t = blockIdx.x; t < b.nptiles; t += gridDim.x) {
@@ -972,7 +971,7 @@ __global__ void __launch_bounds__(kBatchThreads) batch_point_pass_mixed(BatchDev
                     fp64::pass_b_point_rect<true>(b.a, c, cur, ctl.dt, p, tile.nzx, tile.nzy, tile.po,
                                                   4 * (int64_t)tile.zo);
             } else {
-                fp64::pass_b_point_csr<true, kMany>(b.a, c, cur, ctl.dt, p, p < tile.end);
+                fp64::pass_b_point_csr<true, true>(b.a, c, cur, ctl.dt, p, p < tile.end);
             }
         }
     }
@@ -1071,7 +1070,7 @@ cudaError_t launch_batch_pass_a_mixed(const BatchDev& b, bool all_quads, cudaStr
 }
 
 cudaError_t launch_batch_point_pass_mixed(const BatchDev& b, int grid, cudaStream_t stream) {
-    return launch_pdl(b.a.many ? batch_point_pass_mixed<true> : batch_point_pass_mixed<false>, grid, kBatchThreads, 0, stream, b);
+    return launch_pdl(batch_point_pass_mixed, grid, kBatchThreads, 0, stream, b);
 }
 
 cudaError_t prepare_learned_kernels() {
