@@ -58,16 +58,16 @@ MLP_FLOP_PER_ROW = 2 * (16 * 64 + 64 * 64 + 64 * 16)   # tensor-core MMA shapes,
 # DRAM bytes (read + write) of one pass A launch per zone, from the ncu
 # captures of profiles/pass_a_warp_stages_sedov1024.md, 1,048,576 zones
 # each; the bench scales them by its zone count
-PASS_A_TRAFFIC_PER_ZONE = {"learned": (111.112e6 + 77.292e6) / 1048576,
-                           "mixed": (111.099e6 + 78.807e6) / 1048576,
-                           "fp64": (109.265e6 + 121.266e6) / 1048576}
+PASS_A_TRAFFIC_PER_ZONE = {"learned": (111.157e6 + 77.298e6) / 1048576,
+                           "mixed": (111.111e6 + 76.568e6) / 1048576,
+                           "fp64": (109.238e6 + 122.723e6) / 1048576}
 
 
-# FP64 thread-instructions a zone of one FP64 pass A launch (ncu
-# sm__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on, 1024^2 Sedov:
-# profiles/pass_a_warp_stages_sedov1024.md), and the B200's FP64 rate a
+# FP64 thread-instructions a zone of one FP64 pass A launch, comparisons
+# among them (ncu sm__sass_thread_inst_executed_op_fp64_pred_on, 1024^2 Sedov
+# in mid-course: profiles/pass_a_warp_stages_sedov1024.md), and the B200's FP64 rate a
 # clock per SM (sm__sass_thread_inst_executed_op_dfma_pred_on peak)
-FP64_PASS_A_INST_PER_ZONE = 713.6
+FP64_PASS_A_INST_PER_ZONE = 766.5
 FP64_INST_PER_CLOCK_PER_SM = 64
 
 
@@ -769,8 +769,9 @@ def main():
         ach = FP64_PASS_A_INST_PER_ZONE * nz / (ms / 1e3) / 1e12
         return {"bound": "fp64 pipe", "kernel": "pass A (fp64)", "achieved": ach, "peak": peak,
                 "unit": "T FP64 thread-instructions/s", "frac": ach / peak, "launch_ms": ms,
-                "note": "FP64 instructions a zone from profiles/pass_a_warp_stages_sedov1024.md (1024^2 at cycle "
-                        "16000); the count depends on how much of the mesh is quiescent"}
+                "note": "FP64 instructions a zone (all, comparisons among them) from "
+                        "profiles/pass_a_warp_stages_sedov1024.md, a 1024^2 blast in mid-course; the count depends on "
+                        "how many corners compress"}
 
     kms_head = res[args.precision]["kernel_ms"]
     dom = int(np.argmax(kms_head[:3]))

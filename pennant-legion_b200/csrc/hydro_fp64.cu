@@ -17,12 +17,11 @@
 // Passes A and C add their blocks' dt minimum, dV/V maximum and inverted
 // sides to the cycle's reductions with atomics (exact in any order).
 //
-// Pass A runs one thread per zone: the zone's sides in the reference's side
-// order, each zone-level quantity (centre, sums, EOS) formed once, no
-// shuffles, its quotients and roots in straight-line code (ieee_div.cuh).
-// Pass C is the persistent staged kernel of pass_c.cu (one
-// thread per zone, inputs gathered into shared memory by asynchronous
-// copies); the batched kernels run the same two bodies.  1/elen is formed
+// Pass A runs one thread per zone (four lanes a zone on small meshes): the
+// zone's sides in the reference's side order, each zone-level quantity
+// (centre, sums, EOS) formed once, its quotients and roots in straight-line
+// code (ieee_div.cuh).  Pass C is in pass_c.cu.  The batched kernels run the
+// same bodies.  1/elen is formed
 // once per side and shared with the neighbouring corner; QCS terms the
 // reference computes and then discards (evol and du unless cdiv < 0, zkur
 // when cdiv > 0) are not computed, which leaves every stored value
@@ -43,10 +42,11 @@ using namespace fp64;
 // two stages (zone_stage.cuh).  Zones that the straight-line body refuses are noted in
 // a.redo and formed after the loop with the operators, from global memory:
 // inlined into the loop, that body's registers would spill the fast one's.
-// 1920^2 Sedov: 0.38 ms, against 0.515 ms for one zone a thread with plain
+// 1920^2 Sedov: 0.370 ms, against 0.515 ms for one zone a thread with plain
 // loads and the division operator at 16 warps an SM; with this body 0.44 ms
-// at 12 warps and 0.52 ms at 16.  FP64 pipe 54% (its busy time alone is 0.18
-// ms), issue slots 50%.
+// at 12 warps and 0.52 ms at 16.  Its 766 FP64 instructions a zone, comparisons
+// among them, would keep the FP64 pipe busy 0.152 ms; the pipe is active 53% of
+// the time at 1024^2 and the issue slots 46%.
 using zstage::MeshKind;
 using zstage::kGeneral;
 using zstage::kQuads;
