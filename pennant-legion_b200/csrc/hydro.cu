@@ -295,7 +295,7 @@ pnt_status init_hydro(pnt_hydro* h, const Mesh& m, const pnt_params& p) {
     a.nums = (int32_t)ns;
     a.quads = m.all_quads ? 1 : 0;
     a.rect_nzx = m.rect_nzx;
-    for (int64_t q = 0; q < np && !a.many; ++q) a.many = m.poff[q + 1] - m.poff[q] > kManyCorners;
+    for (int64_t q = 0; a.rect_nzx <= 0 && q < np && !a.many; ++q) a.many = m.poff[q + 1] - m.poff[q] > kManyCorners;
     int32_t *zfirst = nullptr, *znump = nullptr, *mapsp1 = nullptr, *poff = nullptr, *pcorner = nullptr;
     double* smf = nullptr;
     uint16_t* mask = nullptr;
