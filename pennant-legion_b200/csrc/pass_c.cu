@@ -197,7 +197,13 @@ __global__ void __launch_bounds__(kSmallThreads) pass_c_small(DevArrays a, Hydro
     const double x0x = a.px[cur][p].x;
     const double2 sf = a.sftot[ix.s0 + k];
     const unsigned mask = a.bcmask[p];
-    const double zm = a.zm[z], zetot0 = a.zetot[z], zvol0 = a.zvol[z], zp = a.zp[z];
+    double zm = 0., zetot0 = 0., zvol0 = 0., zp = 0.;
+    if (live) {   // the last zone's energy and volume may be its own warp's results by now
+        zm = a.zm[z];
+        zetot0 = a.zetot[z];
+        zvol0 = a.zvol[z];
+        zp = a.zp[z];
+    }
     const double dth = 0.5 * dt;
     const double xpx = x0x + u0.x * dth;
     double2 ub = u0;
